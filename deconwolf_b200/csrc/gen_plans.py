@@ -97,31 +97,80 @@ def padn(n, s):
     return n + n // s[0] + 1
 
 
-def x_smem(n, split, R):
-    """Shared memory of k_xpass<RD, R> (mirrors XCfg in passes.cuh)."""
-    a, b, c = split
-    rev = (c, b, a) if c > 1 else (b, a, 1)
-    tpl = max(tpl_of(n, split), tpl_of(n, rev))
-    threads = R * tpl
-    row = max(n + 1, padn(n, split), padn(n, rev)) | 1
-    nkb = (n + 1 + KB - 1) // KB
-    area = (max(R * nkb * KB, R * row) + 1) // 2 * 2
-    return 64 + 8 * area + 3 * 4 * R * ((2 * n + 3) // 4 * 4) + 8 * threads
+def x_fits(n):
+    """Complex half lengths the x pass takes: a CTA with one tile of rows of
+    the best split, staged with three real rows each, fits shared memory."""
+    s = best_split(n)
+    rev = (s[2], s[1], s[0]) if s[2] > 1 else (s[1], s[0], 1)
+    row = max(n + 1, padn(n, s), padn(n, rev)) | 1
+    return 64 + 8 * (row + 1) // 2 * 2 + 12 * ((2 * n + 3) // 4 * 4) + 8 * tpl_of(n, s) <= SMEM_MAX
 
 
-def x_R(n, split):
-    """Rows per x tile (complex half length n).  Two rows share each thread;
-    small rows take more thread rows so that a CTA has a full warp; the tile
-    should let three CTAs share an SM."""
-    a, b, c = split
-    rev = (c, b, a) if c > 1 else (b, a, 1)
-    tpl = max(tpl_of(n, split), tpl_of(n, rev))
-    R = 2
-    while R * tpl < 64:
-        R *= 2
-    while R > 1 and (3 * x_smem(n, split, R) > 225 * 1024 or R * tpl > 1024):
-        R //= 2
-    return R, tpl
+# Issue cost of a radix-r butterfly (about 0.65 of its real additions and
+# multiplications: pairs of them are one instruction, plus register moves)
+DFT_COST = {1: 0, 2: 4, 3: 12, 4: 12, 5: 28, 6: 32, 7: 58, 8: 38, 9: 72, 10: 66, 12: 76, 14: 128, 15: 130, 16: 112}
+
+
+def x_cost(n, s, tp):
+    """Modelled cost per element of the x pass (forward plus inverse) with
+    split s and tp threads per row (xpass.cuh), and the values held per
+    thread.  Each stage's warps issue for their busiest lane; the weights
+    were fitted to measured update and ratio passes of 57 lengths (2 to 13
+    plans each; the plan picked is 2.6 % behind the best measured one on
+    average)."""
+    a, b, c = s
+    three = c > 1
+    last = c if three else b
+    ceil = lambda x, y: -(-x // y)  # noqa: E731
+    m = n // a
+    # (butterflies or pairs, instructions of one, values held)
+    stages = [(ceil(m, 2), 4 * DFT_COST[a] + a * X_W["pair"], 2 * a)]
+    if three:
+        stages.append((n // b, 2 * (DFT_COST[b] + b * X_W["mid"]), b))
+    stages.append((n // last, 2 * DFT_COST[last] + last * X_W["op"], last + 3))  # and the op's operands
+    cost, held = 0.0, 0
+    rowwarps = tp / 32
+    for count, ins, regs in stages:
+        q = ceil(count, tp)
+        held = max(held, q * regs)
+        for i in range(q):
+            active = min(tp, count - i * tp)
+            cost += (ceil(active, 32) if tp >= 32 else rowwarps) * ins
+    cost += (6 if three else 3) * (X_W["sync32"] if tp <= 32 else X_W["sync"]) * rowwarps
+    cost += X_W["row"] * max(1, rowwarps)
+    # fewer resident warps than a scheduler can interleave leave slots empty
+    regs = max(48, 2 * held + 35)
+    threads, rows = (tp, 1) if tp > 32 else (128, 128 // tp)
+    ctas = min(65536 / (regs * ceil(threads, 32) * 32), 227 * 1024 / (rows * 18 * n + 1024))
+    if ctas < 1:
+        return 1e9, held
+    return cost / n / min(1.0, ctas * ceil(threads, 32) / 4 / X_W["latency"]), held
+
+
+X_W = dict(pair=48, mid=11, op=69, sync32=9, sync=30, row=55, latency=8.8)
+
+
+def x_R(tp):
+    """Rows per tile: one CTA has at least 128 threads up to 32 threads per
+    row, two rows above (the error partials are per tile)."""
+    return 2 if tp > 32 else 128 // tp
+
+
+X_TP = [4, 8, 16, 32, 64, 96, 128, 160, 192, 256]
+X_HELD_MAX = 34
+
+
+def x_ranked(n):
+    """(split, TP) of half length n, cheapest by x_cost first."""
+    out = []
+    for s in ranked_splits(n):
+        if s[0] == 1:
+            continue
+        for tp in X_TP:
+            cost, held = x_cost(n, s, tp)
+            if held <= X_HELD_MAX:
+                out.append((cost, s, tp))
+    return [(s, tp) for _, s, tp in sorted(out)]
 
 
 def y_fits(n, split):
@@ -187,9 +236,10 @@ def alternates(n, ok, count):
 #     split at its column tile T, the best alternate split, and the best
 #     split with half the column tile
 #   y (persistent 4-line tiles): the best split and up to two alternates
-#   x: the best split; for half lengths >= X_ALT_MIN one alternate split with
-#     the same rows per tile, compiled for the iteration's two families
-#     (ratio and update) only -- the set-up families use candidate 0
+#   x: the best split and threads per row by a cost model; for half lengths
+#     >= X_ALT_MIN one alternate split with the same rows per tile, compiled
+#     for the iteration's two families (ratio and update) only -- the set-up
+#     families use candidate 0
 X_ALT_MIN = 96
 
 
@@ -210,15 +260,16 @@ def y_cands(n):
 
 
 def x_cands(n):
-    s0 = best_split(n)
-    R0, _ = x_R(n, s0)
-    out = [(s0, R0)]
+    """[(split, TP, R)]: the cheapest by the model; for half lengths >=
+    X_ALT_MIN also the next one with another radix list and the same R."""
+    ranked = x_ranked(n)
+    s0, tp0 = ranked[0]
+    out = [(s0, tp0, x_R(tp0))]
     if n >= X_ALT_MIN:
-        def ok(s):
-            R, _ = x_R(n, s)
-            return R == R0 and x_smem(n, s, R) <= SMEM_MAX
-        for s in alternates(n, ok, 1):
-            out.append((s, R0))
+        for s, tp in ranked[1:]:
+            if s != s0 and x_R(tp) == x_R(tp0):
+                out.append((s, tp, x_R(tp)))
+                break
     return out
 
 
@@ -231,7 +282,7 @@ def main():
     args = ap.parse_args()
 
     lines_ns = supported(args.max, start=1)
-    x_ns = [n for n in supported(args.xmax) if x_smem(n, best_split(n), x_R(n, best_split(n))[0]) <= SMEM_MAX]
+    x_ns = [n for n in supported(args.xmax) if x_fits(n)]
     if args.only:
         keep = {int(v) for v in args.only.split(",")}
         lines_ns = [n for n in lines_ns if n in keep or n == 1]
@@ -241,7 +292,7 @@ def main():
     hdr = []
     hdr.append("// generated by gen_plans.py -- do not edit")
     hdr.append("#pragma once")
-    hdr.append("#include \"passes.cuh\"")
+    hdr.append("#include \"xpass.cuh\"")
     hdr.append("namespace dwcu {")
     hdr.append("// one entry per autotuning candidate of a length, candidates of a length in")
     hdr.append("// order (cand 0: the generator's heuristic choice)")
@@ -265,9 +316,10 @@ def main():
     hdr.append("};")
     hdr.append("static const XPlan kXPlans[] = {")
     for n in x_ns:
-        for c, (s, R) in enumerate(x_cands(n)):
-            hdr.append(f"    {{{n}, {c}, {s[0]}, {s[1]}, {s[2]}, {R}, XCfg<{rad_str(s)}, {R}>::THREADS, "
-                       f"XCfg<{rad_str(s)}, {R}>::SMEM_BYTES, launch_x_{n}_{c}}},")
+        for c, (s, tp, R) in enumerate(x_cands(n)):
+            cfg = f"XCfg<{rad_str(s)}, {tp}, {R}, XFAM_RATIO>"
+            hdr.append(f"    {{{n}, {c}, {s[0]}, {s[1]}, {s[2]}, {R}, {cfg}::THREADS, "
+                       f"{cfg}::SMEM_BYTES, launch_x_{n}_{c}}},")
     hdr.append("};")
     hdr.append("static const YPlan kYPlans[] = {")
     for n in y_ns:
@@ -291,7 +343,7 @@ def main():
             if kind == "y":
                 # the y pass runs faster with scalar complex adds (dft.cuh)
                 lines.append("#define DW_PAIRED_ADDS 0")
-            lines += ["#include \"launch.cuh\"", "namespace dwcu {"]
+            lines += ["#include \"launch_x.cuh\"" if kind == "x" else "#include \"launch.cuh\"", "namespace dwcu {"]
             if kind == "x":
                 lines += [f"void launch_x_{n}_0(const XArgs &, cudaStream_t);" for n in chunk]
             for n in chunk:
@@ -300,13 +352,13 @@ def main():
                         lines.append(f"void launch_lines_{n}_{c}(const LinesArgs &a, int nb, cudaStream_t st) "
                                      f"{{ launch_lines_t<{rad_str(s)}, {T}>(a, nb, st); }}")
                 elif kind == "x":
-                    for c, (s, R) in enumerate(x_cands(n)):
+                    for c, (s, tp, R) in enumerate(x_cands(n)):
                         if c == 0:
                             lines.append(f"void launch_x_{n}_0(const XArgs &a, cudaStream_t st) "
-                                         f"{{ launch_x_t<{rad_str(s)}, {R}>(a, st); }}")
+                                         f"{{ launch_x_t<{rad_str(s)}, {tp}, {R}>(a, st); }}")
                         else:
                             lines.append(f"void launch_x_{n}_{c}(const XArgs &a, cudaStream_t st) "
-                                         f"{{ if (x_iteration_op(a.op)) launch_x_iter_t<{rad_str(s)}, {R}>(a, st); "
+                                         f"{{ if (x_iteration_op(a.op)) launch_x_iter_t<{rad_str(s)}, {tp}, {R}>(a, st); "
                                          f"else launch_x_{n}_0(a, st); }}")
                 else:
                     for c, s in enumerate(y_cands(n)):

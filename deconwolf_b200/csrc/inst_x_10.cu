@@ -1,5 +1,5 @@
 // generated by gen_plans.py -- do not edit
-#include "launch.cuh"
+#include "launch_x.cuh"
 namespace dwcu {
 void launch_x_14_0(const XArgs &, cudaStream_t);
 void launch_x_45_0(const XArgs &, cudaStream_t);
@@ -12,24 +12,24 @@ void launch_x_750_0(const XArgs &, cudaStream_t);
 void launch_x_1008_0(const XArgs &, cudaStream_t);
 void launch_x_1372_0(const XArgs &, cudaStream_t);
 void launch_x_1890_0(const XArgs &, cudaStream_t);
-void launch_x_14_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 2, 1>, 16>(a, st); }
-void launch_x_45_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 5, 1>, 8>(a, st); }
-void launch_x_96_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<12, 8, 1>, 8>(a, st); }
-void launch_x_96_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 12, 1>, 8>(a, st); else launch_x_96_0(a, st); }
-void launch_x_162_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 3, 6>, 2>(a, st); }
-void launch_x_162_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 3, 9>, 2>(a, st); else launch_x_162_0(a, st); }
-void launch_x_252_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 6, 6>, 2>(a, st); }
-void launch_x_252_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 6, 7>, 2>(a, st); else launch_x_252_0(a, st); }
-void launch_x_384_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 6, 8>, 2>(a, st); }
-void launch_x_384_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 8, 8>, 2>(a, st); else launch_x_384_0(a, st); }
-void launch_x_540_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<10, 6, 9>, 2>(a, st); }
-void launch_x_540_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 6, 10>, 2>(a, st); else launch_x_540_0(a, st); }
-void launch_x_750_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<15, 5, 10>, 2>(a, st); }
-void launch_x_750_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<10, 5, 15>, 2>(a, st); else launch_x_750_0(a, st); }
-void launch_x_1008_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<14, 8, 9>, 2>(a, st); }
-void launch_x_1008_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 8, 14>, 2>(a, st); else launch_x_1008_0(a, st); }
-void launch_x_1372_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<14, 7, 14>, 1>(a, st); }
-void launch_x_1372_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 14, 14>, 1>(a, st); else launch_x_1372_0(a, st); }
-void launch_x_1890_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<15, 9, 14>, 1>(a, st); }
-void launch_x_1890_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<14, 9, 15>, 1>(a, st); else launch_x_1890_0(a, st); }
+void launch_x_14_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<2, 7, 1>, 4, 32>(a, st); }
+void launch_x_45_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<3, 5, 3>, 8, 16>(a, st); }
+void launch_x_96_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 1>, 8, 16>(a, st); }
+void launch_x_96_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<2, 4, 12>, 8, 16>(a, st); else launch_x_96_0(a, st); }
+void launch_x_162_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<3, 9, 6>, 32, 4>(a, st); }
+void launch_x_162_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<3, 6, 9>, 32, 4>(a, st); else launch_x_162_0(a, st); }
+void launch_x_252_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 9, 4>, 32, 4>(a, st); }
+void launch_x_252_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<4, 7, 9>, 32, 4>(a, st); else launch_x_252_0(a, st); }
+void launch_x_384_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 4, 12>, 32, 4>(a, st); }
+void launch_x_384_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<2, 16, 12>, 32, 4>(a, st); else launch_x_384_0(a, st); }
+void launch_x_540_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 12, 9>, 64, 2>(a, st); }
+void launch_x_540_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 10, 9>, 64, 2>(a, st); else launch_x_540_0(a, st); }
+void launch_x_750_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 15, 10>, 96, 2>(a, st); }
+void launch_x_750_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 10, 15>, 96, 2>(a, st); else launch_x_750_0(a, st); }
+void launch_x_1008_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<6, 14, 12>, 96, 2>(a, st); }
+void launch_x_1008_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 12, 12>, 96, 2>(a, st); else launch_x_1008_0(a, st); }
+void launch_x_1372_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 14, 14>, 128, 2>(a, st); }
+void launch_x_1372_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<14, 14, 7>, 128, 2>(a, st); else launch_x_1372_0(a, st); }
+void launch_x_1890_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 14, 15>, 160, 2>(a, st); }
+void launch_x_1890_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 15, 14>, 160, 2>(a, st); else launch_x_1890_0(a, st); }
 }  // namespace dwcu

@@ -1,5 +1,5 @@
 // generated by gen_plans.py -- do not edit
-#include "launch.cuh"
+#include "launch_x.cuh"
 namespace dwcu {
 void launch_x_10_0(const XArgs &, cudaStream_t);
 void launch_x_40_0(const XArgs &, cudaStream_t);
@@ -12,22 +12,22 @@ void launch_x_729_0(const XArgs &, cudaStream_t);
 void launch_x_980_0(const XArgs &, cudaStream_t);
 void launch_x_1344_0(const XArgs &, cudaStream_t);
 void launch_x_1792_0(const XArgs &, cudaStream_t);
-void launch_x_10_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 2, 1>, 16>(a, st); }
-void launch_x_40_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 5, 1>, 8>(a, st); }
-void launch_x_84_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<12, 7, 1>, 8>(a, st); }
-void launch_x_150_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<15, 10, 1>, 8>(a, st); }
-void launch_x_150_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<10, 15, 1>, 8>(a, st); else launch_x_150_0(a, st); }
-void launch_x_245_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 5, 7>, 2>(a, st); }
-void launch_x_245_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 7, 7>, 2>(a, st); else launch_x_245_0(a, st); }
-void launch_x_375_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<15, 5, 5>, 2>(a, st); }
-void launch_x_375_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 5, 15>, 2>(a, st); else launch_x_375_0(a, st); }
-void launch_x_512_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 8, 8>, 2>(a, st); }
-void launch_x_512_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<16, 4, 8>, 2>(a, st); else launch_x_512_0(a, st); }
-void launch_x_729_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 9, 9>, 2>(a, st); }
-void launch_x_980_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<14, 7, 10>, 2>(a, st); }
-void launch_x_980_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<10, 7, 14>, 2>(a, st); else launch_x_980_0(a, st); }
-void launch_x_1344_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<14, 8, 12>, 1>(a, st); }
-void launch_x_1344_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<12, 8, 14>, 1>(a, st); else launch_x_1344_0(a, st); }
-void launch_x_1792_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<16, 8, 14>, 1>(a, st); }
-void launch_x_1792_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<14, 8, 16>, 1>(a, st); else launch_x_1792_0(a, st); }
+void launch_x_10_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<2, 5, 1>, 4, 32>(a, st); }
+void launch_x_40_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<2, 2, 10>, 4, 32>(a, st); }
+void launch_x_84_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 12, 1>, 8, 16>(a, st); }
+void launch_x_150_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 3, 10>, 16, 8>(a, st); }
+void launch_x_150_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<3, 5, 10>, 16, 8>(a, st); else launch_x_150_0(a, st); }
+void launch_x_245_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 7, 5>, 32, 4>(a, st); }
+void launch_x_245_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 7, 7>, 32, 4>(a, st); else launch_x_245_0(a, st); }
+void launch_x_375_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 5, 15>, 32, 4>(a, st); }
+void launch_x_375_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 15, 5>, 32, 4>(a, st); else launch_x_375_0(a, st); }
+void launch_x_512_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 8, 8>, 64, 2>(a, st); }
+void launch_x_512_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<4, 16, 8>, 64, 2>(a, st); else launch_x_512_0(a, st); }
+void launch_x_729_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 9, 9>, 96, 2>(a, st); }
+void launch_x_980_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 14, 10>, 128, 2>(a, st); }
+void launch_x_980_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<10, 14, 7>, 96, 2>(a, st); else launch_x_980_0(a, st); }
+void launch_x_1344_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 14>, 128, 2>(a, st); }
+void launch_x_1344_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 12>, 128, 2>(a, st); else launch_x_1344_0(a, st); }
+void launch_x_1792_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 16, 14>, 160, 2>(a, st); }
+void launch_x_1792_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 16>, 128, 2>(a, st); else launch_x_1792_0(a, st); }
 }  // namespace dwcu

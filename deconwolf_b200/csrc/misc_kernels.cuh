@@ -6,7 +6,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
-#include "passes.cuh"
+#include "xpass.cuh"
 
 namespace dwcu {
 
@@ -15,6 +15,7 @@ constexpr int kRedThreads = 256;
 struct StatsPartial {
     double sum;
     float mn;
+    float mx;  // largest magnitude
     int nonfinite;
 };
 
@@ -25,10 +26,10 @@ k_stats_partial(const float *__restrict__ g, long long GP, int M, long long nrow
                 StatsPartial *__restrict__ part)
 {
     __shared__ double ssum[kRedThreads];
-    __shared__ float smin[kRedThreads];
+    __shared__ float smin[kRedThreads], smax[kRedThreads];
     __shared__ int snf[kRedThreads];
     double s = 0.0;
-    float mn = INFINITY;
+    float mn = INFINITY, mx = 0.f;
     int nf = 0;
     const long long r0 = (long long) blockIdx.x * rpb;
     const long long r1 = min(nrows, r0 + rpb);
@@ -39,21 +40,24 @@ k_stats_partial(const float *__restrict__ g, long long GP, int M, long long nrow
             if (!isfinite(v)) nf++;
             s += (double) v;
             mn = fminf(mn, v);
+            mx = fmaxf(mx, fabsf(v));
         }
     }
     ssum[threadIdx.x] = s;
     smin[threadIdx.x] = mn;
+    smax[threadIdx.x] = mx;
     snf[threadIdx.x] = nf;
     __syncthreads();
     for (int o = kRedThreads / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) {
             ssum[threadIdx.x] += ssum[threadIdx.x + o];
             smin[threadIdx.x] = fminf(smin[threadIdx.x], smin[threadIdx.x + o]);
+            smax[threadIdx.x] = fmaxf(smax[threadIdx.x], smax[threadIdx.x + o]);
             snf[threadIdx.x] += snf[threadIdx.x + o];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = StatsPartial{ssum[0], smin[0], snf[0]};
+    if (threadIdx.x == 0) part[blockIdx.x] = StatsPartial{ssum[0], smin[0], smax[0], snf[0]};
 }
 
 // Finish the statistics: bg (method_shb.c:108-117), start value
@@ -63,24 +67,27 @@ k_stats_final(const StatsPartial *__restrict__ part, int nb, JobScalars *sc, int
               unsigned long long wmnp_logical)
 {
     __shared__ double ssum[kRedThreads];
-    __shared__ float smin[kRedThreads];
+    __shared__ float smin[kRedThreads], smax[kRedThreads];
     __shared__ int snf[kRedThreads];
     double s = 0.0;
-    float mn = INFINITY;
+    float mn = INFINITY, mx = 0.f;
     int nf = 0;
     for (int i = threadIdx.x; i < nb; i += kRedThreads) {
         s += part[i].sum;
         mn = fminf(mn, part[i].mn);
+        mx = fmaxf(mx, part[i].mx);
         nf += part[i].nonfinite;
     }
     ssum[threadIdx.x] = s;
     smin[threadIdx.x] = mn;
+    smax[threadIdx.x] = mx;
     snf[threadIdx.x] = nf;
     __syncthreads();
     for (int o = kRedThreads / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) {
             ssum[threadIdx.x] += ssum[threadIdx.x + o];
             smin[threadIdx.x] = fminf(smin[threadIdx.x], smin[threadIdx.x + o]);
+            smax[threadIdx.x] = fmaxf(smax[threadIdx.x], smax[threadIdx.x + o]);
             snf[threadIdx.x] += snf[threadIdx.x + o];
         }
         __syncthreads();
@@ -88,6 +95,7 @@ k_stats_final(const StatsPartial *__restrict__ part, int nb, JobScalars *sc, int
     if (threadIdx.x == 0) {
         float gmin = smin[0];
         sc->gmin = gmin;
+        sc->gmax = smax[0];
         sc->sumg = ssum[0];
         sc->bg = bg_auto ? (gmin < 1e-2f ? 1e-2f : gmin) : bg_user;
         const float sumg = (float) ssum[0];

@@ -520,7 +520,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
     // the parts' statistics, combined in part order (k_stats_final's
     // formulas), go back to every part
     double sumg = 0.0;
-    float gmin = INFINITY;
+    float gmin = INFINITY, gmax = 0.f;
     int flags = 0;
     for (auto &pt : sl->parts) {
         if (!pt.j) continue;
@@ -532,20 +532,23 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
         if (pt.pl > 0) {
             sumg += hs.sumg;
             gmin = std::fmin(gmin, hs.gmin);
+            gmax = std::fmax(gmax, hs.gmax);
         }
     }
     if (sl->local >= 0) {
         // over the processes: the image sum and the parts with non-finite
-        // image or PSF values added, the minimum taken
+        // image or PSF values, or with image values beyond the ratio pass's
+        // usual range (kRatioBig), added; the minimum taken
         SlabPart &me = sl->lead();
-        double v[3] = {sumg, (double) (flags & 1), (double) ((flags >> 1) & 1)};
+        double v[4] = {sumg, (double) (flags & 1), (double) ((flags >> 1) & 1), gmax <= kRatioBig ? 0.0 : 1.0};
         CU(cudaSetDevice(me.device));
         CU(cudaMemcpyAsync(sl->sync_buf, v, sizeof v, cudaMemcpyHostToDevice, me.stream));
-        TRY(slab_sync_allreduce(sl, 3, 0));
+        TRY(slab_sync_allreduce(sl, 4, 0));
         CU(cudaMemcpyAsync(v, sl->sync_buf, sizeof v, cudaMemcpyDeviceToHost, me.stream));
         CU(cudaStreamSynchronize(me.stream));
         sumg = v[0];
         flags = (v[1] > 0 ? 1 : 0) | (v[2] > 0 ? 2 : 0);
+        if (v[3] > 0) gmax = INFINITY;
         double m = (double) gmin;
         CU(cudaMemcpyAsync(sl->sync_buf, &m, sizeof m, cudaMemcpyHostToDevice, me.stream));
         TRY(slab_sync_allreduce(sl, 1, 1));
@@ -571,6 +574,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
     }
     JobScalars all{};
     all.gmin = gmin;
+    all.gmax = gmax;
     all.sumg = sumg;
     all.bg = sl->s.bg_auto ? (gmin < 1e-2f ? 1e-2f : gmin) : sl->s.bg;
     all.x0 = (float) sumg / (float) wmnp;

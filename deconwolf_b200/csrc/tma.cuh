@@ -98,6 +98,14 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// into L2, without waiting: the 32 bytes at p (any alignment) / bytes at p
+// (address and size multiples of 16)
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_l2_bulk(const void *p, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // Bounded wait by one thread for a copy still in flight before an early exit
 // (a CTA must not exit while a bulk copy is writing its shared memory).
 __device__ __forceinline__ void drain(uint64_t *bar, uint32_t parity)
