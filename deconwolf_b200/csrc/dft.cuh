@@ -109,6 +109,16 @@ DW_HD float2 cmulc(float2 a, float2 b)  // a * conj(b)
     return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 #endif
 }
+// the products above in paired instructions whatever the translation unit's
+// DW_PAIRED_ADDS: the OTF multiply rounds alike wherever it is fused
+__device__ __forceinline__ float2 cmul_paired(float2 a, float2 b)
+{
+    return __ffma2_rn(make_float2(-a.y, a.x), make_float2(b.y, b.y), __fmul2_rn(a, make_float2(b.x, b.x)));
+}
+__device__ __forceinline__ float2 cmulc_paired(float2 a, float2 b)
+{
+    return __ffma2_rn(make_float2(a.y, -a.x), make_float2(b.y, b.y), __fmul2_rn(a, make_float2(b.x, b.x)));
+}
 // multiply by DIR*i
 template <int DIR>
 DW_HD float2 mul_i(float2 v)

@@ -577,6 +577,7 @@ struct dwcu_job {
     float *h_err = nullptr;
     cudaEvent_t ev_rb[2] = {nullptr, nullptr};
     int spec = -1;                 // iteration whose forward half is queued ahead of its decision
+    long long x_pitch = 0;         // pitch of the x pass's real rows (0: the geometry's XP)
     long long slab_elems = 0;      // complex elements of each column buffer (0: a whole job)
     bool slab_copies = false;      // the z pass works on gathered copies (T allocated)
     float2 *T = nullptr;
@@ -591,7 +592,7 @@ static int trace_cap(const dwcu_opts &s) { return std::max(1, std::max(s.n_iter,
 static int launch_lines(dwcu_job *j, const LinesPlan *p, const float2 *tw, long long n, long long line_stride,
                         long long outer_stride, long long nouter, long long ncols, int mode, float2 *data,
                         const char *axis, long long nin = -1, long long nout = -1, float2 *const *planes = nullptr,
-                        long long col0 = 0)
+                        long long col0 = 0, float2 *packed = nullptr)
 {
     if (nin < 0) nin = n;
     if (nout < 0) nout = n;
@@ -609,6 +610,12 @@ static int launch_lines(dwcu_job *j, const LinesPlan *p, const float2 *tw, long 
     a.nout = (int) nout;
     a.planes = planes;
     a.col0 = col0;
+    if (packed) {
+        a.packed = packed;
+        a.packed_row = (int) (j->g.X / 2 + 1);
+        a.packed_y = (int) j->g.Y;
+        a.packed_stride = (long long) a.packed_row * a.packed_y;
+    }
     long long nb = (long long) a.ntiles * nouter;
     if (nb > 0x7fffffffLL) return fail(DWCU_ERROR_UNSUPPORTED, "grid too large");
     static const char *names[] = {"lines_fwd", "lines_inv", "lines_conv", "lines_conv_conj"};
@@ -648,13 +655,14 @@ static int pass_y(dwcu_job *j, int mode, float2 *data, long long planes = -1)
     return launch_lines(j, g.yp, j->tw_y, g.Y, KB, g.Y * KB, planes * g.NKB, KB, mode, data, "y");
 }
 // z transforms; planes >= nin are taken as zero and not read, only planes
-// < nout are written (defaults: all)
-static int pass_z(dwcu_job *j, int mode, float2 *data, long long nin = -1, long long nout = -1)
+// < nout are written (defaults: all); packed: see LinesArgs
+static int pass_z(dwcu_job *j, int mode, float2 *data, long long nin = -1, long long nout = -1,
+                  float2 *packed = nullptr)
 {
     const Geometry &g = j->g;
     // lines along z: every (kx block, y, kx) of a plane is a column; stride = plane
     const long long plane = g.NKB * g.Y * KB;
-    return launch_lines(j, g.zp, j->tw_z, g.Z, plane, 0, 1, plane, mode, data, "z", nin, nout);
+    return launch_lines(j, g.zp, j->tw_z, g.Z, plane, 0, 1, plane, mode, data, "z", nin, nout, nullptr, 0, packed);
 }
 
 static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, const float *srcp, float *dst,
@@ -673,7 +681,8 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
     a.partial = j->partial;
     a.sc = j->sc;
     a.err = &j->sc->flags;
-    a.X = g.XP;
+    a.X = j->x_pitch ? j->x_pitch : g.XP;
+    a.bulk = a.X % 4 == 0 && (((uintptr_t) src | (uintptr_t) srcp | (uintptr_t) j->W) & 15) == 0;
     a.GP = g.GP;
     a.nkb = (int) g.NKB;
     a.ntiles = (int) (tiles < 0 ? j->nxb : tiles);
@@ -752,8 +761,28 @@ static double shb_alpha(int k, float alphamax)
     return a;
 }
 
+// the convolution of a single plane in one kernel (k_yconv) where its tiles fit
+static bool one_plane(const Geometry &g) { return g.Z == 1 && g.ytp; }
+static int pass_yconv(dwcu_job *j, int conj)
+{
+    const Geometry &g = j->g;
+    YArgs a;
+    a.data = j->S;
+    a.tw = j->tw_y;
+    a.err = &j->sc->flags;
+    a.ntiles = (int) g.NKB;
+    a.dir = 0;
+    a.otf = j->K;
+    a.conj = conj;
+    ProfScope ps(conj ? "y_conv_conj" : "y_conv", 24.0 * (double) g.NKB * KB * g.Y, j->stream);
+    g.ytp->launch(a, j->stream);
+    CHECK_LAUNCH();
+    return DWCU_SUCCESS;
+}
+
 static int conv(dwcu_job *j, int conj)
 {
+    if (one_plane(j->g)) return pass_yconv(j, conj);
     TRY(pass_y(j, LINES_FWD, j->S));
     TRY(pass_z(j, conj ? LINES_CONV_CONJ : LINES_CONV, j->S));
     TRY(pass_y(j, LINES_INV, j->S));
@@ -770,6 +799,7 @@ static int conv(dwcu_job *j, int conj)
 static int conv_forward(dwcu_job *j)
 {
     const Geometry &g = j->g;
+    if (one_plane(g)) return pass_yconv(j, 0);
     TRY(pass_y(j, LINES_FWD, j->S));
     TRY(pass_z(j, LINES_CONV, j->S, g.Z, g.P));
     TRY(pass_y(j, LINES_INV, j->S, g.P));
@@ -779,7 +809,7 @@ static int conv_backward(dwcu_job *j)
 {
     const Geometry &g = j->g;
     // (a periodic z copies image planes into its margins: no zero planes)
-    if (j->s.method != DWCU_METHOD_SHB || g.wz) return conv(j, 1);
+    if (j->s.method != DWCU_METHOD_SHB || g.wz || one_plane(g)) return conv(j, 1);
     TRY(pass_y(j, LINES_FWD, j->S, g.P));
     TRY(pass_z(j, LINES_CONV_CONJ, j->S, g.P, g.Z));
     TRY(pass_y(j, LINES_INV, j->S));
@@ -1719,17 +1749,9 @@ static int one_call(const float *im, long long M, long long N, long long P, cons
     return rc;
 }
 
-// standalone 3-D transforms on exact sizes (fft.c's fft()/ifft())
-static int fft3d(const float *d_in, long long M, long long N, long long P, float *d_out, int device,
-                 cudaStream_t stream, bool forward)
+// a job that only carries a standalone transform's sizes and plans
+static int fft3d_geometry(dwcu_job *j, long long M, long long N, long long P)
 {
-    if (!d_in || !d_out) return fail(DWCU_ERROR_INVALID_VALUE, "NULL argument");
-    if (M < 2 || N < 1 || P < 1 || (M % 2)) return fail(DWCU_ERROR_INVALID_VALUE, "M must be even and >= 2");
-    DeviceCtx *ctx = nullptr;
-    TRY(get_ctx(device, &ctx));
-    CU(cudaSetDevice(device));
-    dwcu_job jj{};
-    dwcu_job *j = &jj;
     dwcu_opts_init(&j->s);
     Geometry &g = j->g;
     g.M = M; g.N = N; g.P = P; g.pM = g.pN = g.pP = 1;
@@ -1745,66 +1767,95 @@ static int fft3d(const float *d_in, long long M, long long N, long long P, float
     g.GP = (M + 3) & ~3LL;
     j->s.metric = DWCU_METRIC_IDIV;
     j->s.positivity = 1;
+    j->nxb = x_blocks(g);
+    return DWCU_SUCCESS;
+}
+
+// The x pass reads and writes real rows of any even pitch where they start
+// at multiples of 8 bytes, so the caller's volume is used where it lies; one
+// at an odd float goes through `real` (XP-pitched).
+static bool x_takes(const float *p) { return ((uintptr_t) p & 7) == 0; }
+
+static int fft3d_forward(dwcu_job *j, const float *d_in, float *d_out, float *real)
+{
+    const Geometry &g = j->g;
+    const float *src = d_in;
+    j->x_pitch = g.M;
+    if (!x_takes(d_in)) {
+        CU(cudaMemcpy2DAsync(real, sizeof(float) * g.XP, d_in, sizeof(float) * g.M, sizeof(float) * g.M, g.N * g.P,
+                             cudaMemcpyDeviceToDevice, j->stream));
+        src = real;
+        j->x_pitch = g.XP;
+    }
+    TRY(pass_x(j, XOP_FWD_COPY, 1, j->S, src, nullptr, nullptr, 0, 0));
+    TRY(pass_y(j, LINES_FWD, j->S));
+    return pass_z(j, LINES_FWD, j->S, -1, -1, reinterpret_cast<float2 *>(d_out));
+}
+
+static int fft3d_inverse(dwcu_job *j, const float *d_in, float *d_out, float *real)
+{
+    const Geometry &g = j->g;
+    const bool direct = x_takes(d_out);
+    j->x_pitch = direct ? g.M : g.XP;
+    TRY(pass_z(j, LINES_INV, j->S, -1, -1, reinterpret_cast<float2 *>(const_cast<float *>(d_in))));
+    TRY(pass_y(j, LINES_INV, j->S));
+    TRY(pass_x(j, XOP_STORE, 0, j->S, nullptr, nullptr, direct ? d_out : real, 0, 0));
+    if (!direct)
+        CU(cudaMemcpy2DAsync(d_out, sizeof(float) * g.M, real, sizeof(float) * g.XP, sizeof(float) * g.M, g.N * g.P,
+                             cudaMemcpyDeviceToDevice, j->stream));
+    return DWCU_SUCCESS;
+}
+
+// waits for the transform and reports a pass's bounded wait that gave up
+static int fft3d_finish(dwcu_job *j, int rc)
+{
+    JobScalars hs{};
+    cudaError_t e = cudaMemcpyAsync(&hs, j->sc, sizeof hs, cudaMemcpyDeviceToHost, j->stream);
+    const cudaError_t es = cudaStreamSynchronize(j->stream);
+    if (e == cudaSuccess) e = es;
+    if (rc != DWCU_SUCCESS) return rc;
+    if (e != cudaSuccess) return fail(DWCU_ERROR_CUDA, "transform failed: %s", cudaGetErrorString(e));
+    if (hs.flags & ~3) return fail(DWCU_ERROR_TIMEOUT, "a bounded wait in a pass gave up (flags 0x%x)", hs.flags);
+    return DWCU_SUCCESS;
+}
+
+// Standalone 3-D transforms on exact sizes (fft.c's fft()/ifft()): three
+// passes, x on the caller's real volume and z on its half-spectrum, with the
+// blocked spectrum between them in a cached memory block (an allocation and
+// its release cost more than the transform of a 512 x 512 x 60 volume).
+// Spectrum columns past X/2 are transformed along and never read out.
+static int fft3d(const float *d_in, long long M, long long N, long long P, float *d_out, int device,
+                 cudaStream_t stream, bool forward)
+{
+    if (!d_in || !d_out) return fail(DWCU_ERROR_INVALID_VALUE, "NULL argument");
+    if (M < 2 || N < 1 || P < 1 || (M % 2)) return fail(DWCU_ERROR_INVALID_VALUE, "M must be even and >= 2");
+    DeviceCtx *ctx = nullptr;
+    TRY(get_ctx(device, &ctx));
+    CU(cudaSetDevice(device));
+    dwcu_job jj{};
+    dwcu_job *j = &jj;
+    TRY(fft3d_geometry(j, M, N, P));
+    const Geometry &g = j->g;
     j->ctx = ctx;
     j->stream = stream ? stream : ctx->stream;
-    j->nxb = x_blocks(g);
     TRY(get_twiddles(ctx, g.X, &j->tw_x));
     TRY(get_twiddles(ctx, g.X / 2, &j->tw_l));
     if (N > 1) TRY(get_twiddles(ctx, N, &j->tw_y));
     TRY(get_twiddles(ctx, P, &j->tw_z));
     const size_t C = align256(sizeof(float2) * (size_t) (g.spec_elems() + 8 * KB));
-    const size_t R = align256(sizeof(float) * (size_t) (g.real_elems() + g.XP));
-    void *tmp = nullptr;
-    CU(cudaMalloc(&tmp, C + R + 256));
-    j->S = (float2 *) tmp;
-    float *real = (float *) ((char *) tmp + C);
-    j->sc = (JobScalars *) ((char *) tmp + C + R);
-    j->K = nullptr;
-    j->W = nullptr;
-    j->partial = nullptr;
+    const size_t R = x_takes(forward ? d_in : d_out) ? 0 : align256(sizeof(float) * (size_t) (g.real_elems() + g.XP));
+    Block *blk = block_get(device, C + R + 256);
+    if (!blk) return fail(DWCU_ERROR_OUT_OF_MEMORY, "cudaMalloc of %.3f GB for a transform failed", (C + R) / 1e9);
+    j->S = (float2 *) blk->ptr;
+    float *real = (float *) (blk->ptr + C);
+    j->sc = (JobScalars *) (blk->ptr + C + R);
     int rc = DWCU_SUCCESS;
-    const long long H = M / 2 + 1;
-    const long long nspec = H * N * P;
-    const int fb = (int) std::min<long long>(148 * 16, (nspec + 255) / 256);
-    if (cudaMemsetAsync(tmp, 0, C + R + 256, j->stream) != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "memset");
-    if (forward) {
-        if (rc == DWCU_SUCCESS &&
-            cudaMemcpy2DAsync(real, sizeof(float) * g.XP, d_in, sizeof(float) * M, sizeof(float) * M, N * P,
-                              cudaMemcpyDeviceToDevice, j->stream) != cudaSuccess)
-            rc = fail(DWCU_ERROR_CUDA, "copy failed");
-        if (rc == DWCU_SUCCESS) rc = pass_x(j, XOP_FWD_COPY, 1, j->S, real, nullptr, nullptr, 0, 0);
-        if (rc == DWCU_SUCCESS) rc = pass_y(j, LINES_FWD, j->S);
-        if (rc == DWCU_SUCCESS) rc = pass_z(j, LINES_FWD, j->S);
-        if (rc == DWCU_SUCCESS) {
-            k_spec_unpack<<<fb, 256, 0, j->stream>>>(j->S, (int) H, (int) N, (int) P, (int) g.NKB,
-                                                     reinterpret_cast<float2 *>(d_out));
-            ++g_launches;
-            if (cudaGetLastError() != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "unpack launch failed");
-        }
-    } else {
-        k_spec_pack<<<fb, 256, 0, j->stream>>>(reinterpret_cast<const float2 *>(d_in), (int) H, (int) N, (int) P,
-                                               (int) g.NKB, j->S);
-        ++g_launches;
-        if (cudaGetLastError() != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "pack launch failed");
-        if (rc == DWCU_SUCCESS) rc = pass_z(j, LINES_INV, j->S);
-        if (rc == DWCU_SUCCESS) rc = pass_y(j, LINES_INV, j->S);
-        if (rc == DWCU_SUCCESS) rc = pass_x(j, XOP_STORE, 0, j->S, nullptr, nullptr, real, 0, 0);
-        if (rc == DWCU_SUCCESS &&
-            cudaMemcpy2DAsync(d_out, sizeof(float) * M, real, sizeof(float) * g.XP, sizeof(float) * M, N * P,
-                              cudaMemcpyDeviceToDevice, j->stream) != cudaSuccess)
-            rc = fail(DWCU_ERROR_CUDA, "copy failed");
-    }
-    cudaError_t e = cudaStreamSynchronize(j->stream);
-    JobScalars hs{};
-    if (e == cudaSuccess) e = cudaMemcpy(&hs, j->sc, sizeof hs, cudaMemcpyDeviceToHost);
-    cudaFree(tmp);
-    j->base = nullptr;
-    j->ev0 = j->ev1 = j->ev2 = nullptr;
+    if (cudaMemsetAsync(j->sc, 0, sizeof(JobScalars), j->stream) != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "memset");
+    if (rc == DWCU_SUCCESS) rc = forward ? fft3d_forward(j, d_in, d_out, real) : fft3d_inverse(j, d_in, d_out, real);
+    rc = fft3d_finish(j, rc);
+    block_put(blk);
     j->stream = nullptr;
-    if (rc != DWCU_SUCCESS) return rc;
-    if (e != cudaSuccess) return fail(DWCU_ERROR_CUDA, "transform failed: %s", cudaGetErrorString(e));
-    if (hs.flags & ~3) return fail(DWCU_ERROR_TIMEOUT, "a bounded wait in a pass gave up (flags 0x%x)", hs.flags);
-    return DWCU_SUCCESS;
+    return rc;
 }
 
 // ---- the R2C transform of fft3d on caller-provided device memory (used by
@@ -1830,53 +1881,17 @@ int fft3d_r2c_scratch(const float *d_in, long long M, long long N, long long P, 
 {
     dwcu_job jj{};
     dwcu_job *j = &jj;
-    dwcu_opts_init(&j->s);
-    Geometry &g = j->g;
-    g.M = M; g.N = N; g.P = P; g.pM = g.pN = g.pP = 1;
-    g.wM = g.X = M; g.wN = g.Y = N; g.wP = g.Z = P;
-    g.xp = find_x((int) (M / 2));
-    g.yp = N > 1 ? find_lines((int) N) : nullptr;
-    g.zp = find_lines((int) P);
-    g.ytp = N > 1 ? find_y((int) N) : nullptr;
-    if (!g.xp || (N > 1 && !g.yp) || !g.zp)
-        return fail(DWCU_ERROR_UNSUPPORTED, "unsupported transform size %lld x %lld x %lld", M, N, P);
-    g.XP = (M + 3) & ~3LL;
-    g.NKB = (M / 2 + 1 + KB - 1) / KB;
-    g.GP = (M + 3) & ~3LL;
-    j->s.metric = DWCU_METRIC_IDIV;
-    j->s.positivity = 1;
+    TRY(fft3d_geometry(j, M, N, P));
     j->stream = stream;
-    j->nxb = x_blocks(g);
     j->tw_x = tw[0];
     j->tw_l = tw[1];
     j->tw_y = tw[2];
     j->tw_z = tw[3];
     j->S = S;
     j->sc = sc;
-    const long long H = M / 2 + 1;
-    const long long nspec = H * N * P;
-    const int fb = (int) std::min<long long>(148 * 16, (nspec + 255) / 256);
-    int rc = DWCU_SUCCESS;
-    if (cudaMemcpy2DAsync(real, sizeof(float) * g.XP, d_in, sizeof(float) * M, sizeof(float) * M, N * P,
-                          cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
-        rc = fail(DWCU_ERROR_CUDA, "copy failed");
-    if (rc == DWCU_SUCCESS) rc = pass_x(j, XOP_FWD_COPY, 1, j->S, real, nullptr, nullptr, 0, 0);
-    if (rc == DWCU_SUCCESS) rc = pass_y(j, LINES_FWD, j->S);
-    if (rc == DWCU_SUCCESS) rc = pass_z(j, LINES_FWD, j->S);
-    if (rc == DWCU_SUCCESS) {
-        k_spec_unpack<<<fb, 256, 0, stream>>>(j->S, (int) H, (int) N, (int) P, (int) g.NKB,
-                                               reinterpret_cast<float2 *>(d_out));
-        ++g_launches;
-        if (cudaGetLastError() != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "unpack launch failed");
-    }
-    cudaError_t e = cudaStreamSynchronize(stream);
-    JobScalars hs{};
-    if (e == cudaSuccess) e = cudaMemcpy(&hs, sc, sizeof hs, cudaMemcpyDeviceToHost);
+    const int rc = fft3d_finish(j, fft3d_forward(j, d_in, d_out, real));
     j->stream = nullptr;
-    if (rc != DWCU_SUCCESS) return rc;
-    if (e != cudaSuccess) return fail(DWCU_ERROR_CUDA, "transform failed: %s", cudaGetErrorString(e));
-    if (hs.flags & ~3) return fail(DWCU_ERROR_TIMEOUT, "a bounded wait in a pass gave up (flags 0x%x)", hs.flags);
-    return DWCU_SUCCESS;
+    return rc;
 }
 
 }  // namespace dwcu

@@ -361,9 +361,11 @@ def main():
                                          f"{{ if (x_iteration_op(a.op)) launch_x_iter_t<{rad_str(s)}, {tp}, {R}>(a, st); "
                                          f"else launch_x_{n}_0(a, st); }}")
                 else:
+                    # the convolution of single planes is compiled for candidate 0
                     for c, s in enumerate(y_cands(n)):
+                        conv = f"launch_yconv_t<{rad_str(s)}>(a, st)" if c == 0 else f"launch_y_{n}_0(a, st)"
                         lines.append(f"void launch_y_{n}_{c}(const YArgs &a, cudaStream_t st) "
-                                     f"{{ launch_y_t<{rad_str(s)}>(a, st); }}")
+                                     f"{{ if (a.otf) {conv}; else launch_y_t<{rad_str(s)}>(a, st); }}")
             lines.append("}  // namespace dwcu")
             with open(os.path.join(HERE, f"inst_{kind}_{p}.cu"), "w") as f:
                 f.write("\n".join(lines) + "\n")

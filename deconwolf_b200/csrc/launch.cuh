@@ -52,7 +52,7 @@ void launch_lines_t(const LinesArgs &a, int nblocks, cudaStream_t st)
     using C = LinesCfg<RD, T>;
     constexpr int tpl = C::THREADS / T;
     const size_t smem = a.mode >= LINES_CONV ? C::SMEM_BYTES : C::SMEM_FFT;
-    if (a.planes) {
+    if (a.planes || a.packed) {
         ensure_smem(kp, k_lines<RD, T, true>, C::SMEM_BYTES);
         k_lines<RD, T, true><<<nblocks, dim3(T, tpl), smem, st>>>(a);
     } else {
@@ -78,6 +78,15 @@ void launch_y_t(const YArgs &a, cudaStream_t st)
         launch_y_dir<RD, -1>(a, st);
     else
         launch_y_dir<RD, +1>(a, st);
+}
+
+template <class RD>
+void launch_yconv_t(const YArgs &a, cudaStream_t st)
+{
+    static KernelOnce ko;
+    using C = YConvCfg<RD>;
+    ensure_smem(ko, k_yconv<RD>, C::SMEM_BYTES);
+    k_yconv<RD><<<a.ntiles, dim3(KB, C::TPL), C::SMEM_BYTES, st>>>(a);
 }
 
 }  // namespace dwcu

@@ -305,33 +305,6 @@ __global__ void k_crop(const float *__restrict__ x, int X, int Y, int M, int N, 
     }
 }
 
-// compact half-spectrum (kx fastest, H = X/2+1 per row) <-> blocked layout
-__global__ void k_spec_unpack(const float2 *__restrict__ S, int H, int Y, int Z, int nkb, float2 *__restrict__ out)
-{
-    const long long n = (long long) H * Y * Z;
-    for (long long k = blockIdx.x * (long long) blockDim.x + threadIdx.x; k < n;
-         k += (long long) gridDim.x * blockDim.x) {
-        const int kx = (int) (k % H);
-        const long long r = k / H;
-        const int y = (int) (r % Y);
-        const int z = (int) (r / Y);
-        out[k] = S[(((long long) z * nkb + kx / KB) * Y + y) * KB + kx % KB];
-    }
-}
-
-__global__ void k_spec_pack(const float2 *__restrict__ in, int H, int Y, int Z, int nkb, float2 *__restrict__ S)
-{
-    const long long n = (long long) H * Y * Z;
-    for (long long k = blockIdx.x * (long long) blockDim.x + threadIdx.x; k < n;
-         k += (long long) gridDim.x * blockDim.x) {
-        const int kx = (int) (k % H);
-        const long long r = k / H;
-        const int y = (int) (r % Y);
-        const int z = (int) (r / Y);
-        S[(((long long) z * nkb + kx / KB) * Y + y) * KB + kx % KB] = in[k];
-    }
-}
-
 // finish one iteration's error: mean over the image of the x-pass partials
 // (get_fIdiv dw.c:1492-1524 / get_fMSE dw.c:1461-1490)
 __global__ void __launch_bounds__(kRedThreads)

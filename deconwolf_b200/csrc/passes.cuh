@@ -200,6 +200,15 @@ __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o
 template <class RD>
 using RevRad = Rad<(RD::THREE ? RD::RC : RD::RB), (RD::THREE ? RD::RB : RD::RA), (RD::THREE ? RD::RA : 1)>;
 
+// ------------------------------------------------------------ spectrum layout
+//
+// The half-spectrum (kx < X/2+1) is stored blocked by KB = 4 along kx:
+//   element (kx, y, z) at  ((z * nkb + kx / KB) * Y + y) * KB + kx % KB
+// (nkb = ceil((X/2+1) / KB)).  A y line group (4 neighbouring kx) is then one
+// contiguous Y*32-byte block, a z line is strided by the plane size, and the
+// two rows y, y+1 of one kx block are 64 contiguous bytes for the x pass.
+constexpr int KB = 4;
+
 // ------------------------------------------------------------ k_lines
 
 enum LinesMode { LINES_FWD = 0, LINES_INV = 1, LINES_CONV = 2, LINES_CONV_CONJ = 3 };
@@ -220,6 +229,14 @@ struct LinesArgs {
     // loads and stores); `data` is unused and `line_stride` is the OTF's
     float2 *const *planes = nullptr;
     long long col0 = 0;
+    // packed mode (the standalone transforms' last or first pass): a forward
+    // pass writes, an inverse pass reads, element n of the column (kx, y) at
+    // packed[n * packed_stride + y * packed_row + kx], kx < packed_row: the
+    // caller's plain half-spectrum, with no pass of its own to reorder it
+    float2 *packed = nullptr;
+    long long packed_stride = 0;
+    int packed_row = 0;
+    int packed_y = 0;  // rows per plane
 };
 
 template <class RD, int T>
@@ -236,6 +253,7 @@ struct LinesCfg {
         : (THREADS * 2 <= 1024 && SMEM_BYTES * 2 <= 225 * 1024) ? 2 : 1;
 };
 
+// PL: planes or packed mode
 template <class RD, int T, bool PL = false>
 __global__ void __launch_bounds__(LinesCfg<RD, T>::THREADS, LinesCfg<RD, T>::MIN_BLOCKS)
 k_lines(LinesArgs a)
@@ -252,14 +270,27 @@ k_lines(LinesArgs a)
     const long long off = outer * a.outer_stride + col;
     float2 *base = a.data + off;
     const long long ls = a.line_stride;
-    // element n of this thread's line
-    auto elem = [&](int n) -> float2 * {
-        if constexpr (PL)
-            return a.planes[n] + (a.col0 + col);
-        else
-            return base + (long long) n * ls;
-    };
     const int mode = a.mode;
+    // the packed half-spectrum's element 0 of this line, and whether it has one
+    float2 *pk = nullptr;
+    bool pk_in = false, pk_out = false, valid_in = valid, valid_out = valid;
+    if constexpr (PL) {
+        if (a.packed) {
+            const int q = col / KB, kb = q / a.packed_y, kx = kb * KB + col % KB;
+            pk = a.packed + (long long) (q - kb * a.packed_y) * a.packed_row + kx;
+            pk_in = mode == LINES_INV;
+            pk_out = !pk_in;
+            if (kx >= a.packed_row) (pk_in ? valid_in : valid_out) = false;
+        }
+    }
+    // element n of this thread's line
+    auto elem = [&](int n, bool packed) -> float2 * {
+        if constexpr (PL) {
+            if (a.planes) return a.planes[n] + (a.col0 + col);
+            if (packed) return pk + (long long) n * a.packed_stride;
+        }
+        return base + (long long) n * ls;
+    };
     auto smem = [&](int, int i) { return sm + (size_t) i * T + line; };
     using Cfg = LinesCfg<RD, T>;
     float2 *sotf = sm + Cfg::XCH_F2;  // OTF tile [n][col] (convolve modes)
@@ -282,7 +313,7 @@ k_lines(LinesArgs a)
 #pragma unroll
         for (int r = 0; r < RD::RA; ++r) {
             const int n = t + r * (N / RD::RA);
-            v[0][r] = (valid && n < a.nin) ? *elem(n) : make_float2(0.f, 0.f);
+            v[0][r] = (valid_in && n < a.nin) ? *elem(n, pk_in) : make_float2(0.f, 0.f);
         }
     }
     float2 o[1][RD::RL];
@@ -292,10 +323,10 @@ k_lines(LinesArgs a)
         line_fft<RD, -1, 1>(v, o, t, a.tw, smem);
     constexpr int SL = N / RD::RL;
     if (mode == LINES_FWD || mode == LINES_INV) {
-        if (t < SL && valid) {
+        if (t < SL && valid_out) {
 #pragma unroll
             for (int r = 0; r < RD::RL; ++r)
-                if (t + r * SL < a.nout) *elem(t + r * SL) = o[0][r];
+                if (t + r * SL < a.nout) *elem(t + r * SL, pk_out) = o[0][r];
         }
         return;
     }
@@ -325,18 +356,9 @@ k_lines(LinesArgs a)
     if (t < SQ && valid) {
 #pragma unroll
         for (int r = 0; r < RV::RL; ++r)
-            if (t + r * SQ < a.nout) *elem(t + r * SQ) = q[0][r];
+            if (t + r * SQ < a.nout) *elem(t + r * SQ, false) = q[0][r];
     }
 }
-
-// ------------------------------------------------------------ spectrum layout
-//
-// The half-spectrum (kx < X/2+1) is stored blocked by KB = 4 along kx:
-//   element (kx, y, z) at  ((z * nkb + kx / KB) * Y + y) * KB + kx % KB
-// (nkb = ceil((X/2+1) / KB)).  A y line group (4 neighbouring kx) is then one
-// contiguous Y*32-byte block, a z line is strided by the plane size, and the
-// two rows y, y+1 of one kx block are 64 contiguous bytes for the x pass.
-constexpr int KB = 4;
 
 // ------------------------------------------------------------ k_ypass
 
@@ -346,6 +368,8 @@ struct YArgs {
     int *err;           // error flags (bounded waits)
     int ntiles;         // Z * nkb
     int dir;            // -1 forward, +1 inverse
+    const float2 *otf = nullptr;  // convolution (k_yconv): the OTF, same layout as data
+    int conj = 0;       // multiply by its conjugate
 };
 
 template <class RD>
@@ -438,6 +462,77 @@ k_ypass(YArgs a)
 #pragma unroll
                 for (int q = 0; q < Q; ++q) dst[(size_t) (t + r * SL) * KB + q] = o[q][r];
         }
+    }
+}
+
+// ------------------------------------------------------------ k_yconv
+//
+// The convolution of a job of one plane (Z = 1: no z transform): forward y
+// transform, OTF multiply and inverse y transform of one tile in one kernel,
+// instead of a y pass, a z pass that only multiplies, and a y pass.  One CTA
+// per tile (a plane has at most a few hundred); the OTF's elements, which sit
+// where the forward transform leaves its outputs, are loaded ahead of it.
+// 980 x 768 plane: 35 -> 11 us per convolution.
+template <class RD>
+struct YConvCfg {
+    using RV = RevRad<RD>;
+    static constexpr int TPL = cmax(RD::TPL, RV::TPL);
+    static constexpr int THREADS = KB * TPL;
+    static constexpr int BUF_F2 = cmax(RD::PADN, RV::PADN) * KB;
+    static constexpr size_t SMEM_BYTES = 2 * sizeof(float2) * (size_t) BUF_F2 + 64;
+    static constexpr uint32_t TILE_BYTES = (uint32_t) (RD::N * KB * sizeof(float2));
+};
+
+template <class RD>
+__global__ void __launch_bounds__(YConvCfg<RD>::THREADS)
+k_yconv(YArgs a)
+{
+    using C = YConvCfg<RD>;
+    using RV = RevRad<RD>;
+    constexpr int N = RD::N, SL = N / RD::RL, SQ = N / RV::RL;
+    extern __shared__ __align__(128) unsigned char ysm[];
+    uint64_t *bar = reinterpret_cast<uint64_t *>(ysm);
+    float2 *A = reinterpret_cast<float2 *>(ysm + 64), *B = A + C::BUF_F2;
+    const int l = threadIdx.x, t = threadIdx.y;
+    float2 *tile = a.data + (size_t) blockIdx.x * N * KB;
+    if (t == 0 && l == 0) {
+        mbar_init(bar, 1);
+        fence_mbar_init();
+        mbar_arrive_expect_tx(bar, C::TILE_BYTES);
+        tma_load_1d(A, tile, C::TILE_BYTES, bar);
+    }
+    float2 h[RD::RL];
+    if (t < SL) {
+        const float2 *src = a.otf + (size_t) blockIdx.x * N * KB + l;
+#pragma unroll
+        for (int r = 0; r < RD::RL; ++r) h[r] = __ldg(&src[(size_t) (t + r * SL) * KB]);
+    }
+    __syncthreads();  // the barrier is initialised
+    if (!wait_all(bar, 0, a.err, 1 << 8)) {
+        if (t == 0 && l == 0) drain(bar, 0);
+        return;
+    }
+    auto inA = [&](int, int i) { return A + (size_t) i * KB + l; };
+    auto inB = [&](int, int i) { return B + (size_t) i * KB + l; };
+    float2 v[1][RD::RA], o[1][RD::RL], q[1][RV::RL];
+    if (t < N / RD::RA) {
+#pragma unroll
+        for (int r = 0; r < RD::RA; ++r) v[0][r] = A[(size_t) (t + r * (N / RD::RA)) * KB + l];
+    }
+    // three stages: B, then A; the inverse's first stage writes B again while
+    // the forward's last may still read A.  Two stages: B, then A.
+    line_fft_impl<RD, -1, 1, false, true, decltype(inB), decltype(inA)>(v, o, t, a.tw, inB, inA);
+    if (t < SL) {
+#pragma unroll
+        for (int r = 0; r < RD::RL; ++r) o[0][r] = a.conj ? cmulc_paired(o[0][r], h[r]) : cmul_paired(o[0][r], h[r]);
+    }
+    if constexpr (RD::THREE)
+        line_fft_impl<RV, +1, 1, false, true, decltype(inB), decltype(inA)>(o, q, t, a.tw, inB, inA);
+    else
+        line_fft_impl<RV, +1, 1, false, true, decltype(inA), decltype(inB)>(o, q, t, a.tw, inA, inB);
+    if (t < SQ) {
+#pragma unroll
+        for (int r = 0; r < RV::RL; ++r) tile[(size_t) (t + r * SQ) * KB + l] = q[0][r];
     }
 }
 

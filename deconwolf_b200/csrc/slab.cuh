@@ -378,6 +378,11 @@ static int slab_zpass(dwcu_slab *sl, SlabPart &pt, int mode, float2 *data, long 
 static int slab_conv(dwcu_slab *sl, int conj, bool in_img, bool out_img)
 {
     const Geometry &g = sl->g;
+    if (one_plane(g) && sl->parts.size() == 1 && sl->parts[0].j) {
+        // the whole job in one part: its convolution, rounded as it rounds
+        CU(cudaSetDevice(sl->parts[0].device));
+        return conv(sl->parts[0].j, conj);
+    }
     for (auto &pt : sl->parts) {
         if (!pt.j) continue;
         CU(cudaSetDevice(pt.device));

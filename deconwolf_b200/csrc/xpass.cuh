@@ -42,7 +42,8 @@ struct XArgs {
     double *partial;       // per-tile error partials (ops with an error)
     const JobScalars *sc;  // bg, ...
     int *err;              // error flags (bounded waits)
-    long long X;           // real row pitch (= real length), multiple of 4
+    long long X;           // real row pitch in floats (even)
+    int bulk;              // real rows start at multiples of 16 bytes, X a multiple of 4
     long long GP;          // image row pitch, multiple of 4
     int Y, Z;              // padded dims
     int M, N, P;           // image dims
@@ -450,7 +451,6 @@ struct XCfg {
     using XL = XLine<RD, TP>;
     static constexpr int L = RD::N;
     static constexpr int X = 2 * L;
-    static constexpr int XP = (X + 3) / 4 * 4;  // real row pitch (16-byte rows for bulk copies)
     static constexpr int NKB = (L + 1 + KB - 1) / KB;
     static constexpr int THREADS = R * TP;
     static constexpr size_t ROW_BYTES = sizeof(float2) * (size_t) XL::ROW_F2;
@@ -532,7 +532,7 @@ k_xpass(XArgs a)
 {
     using C = XCfg<RD, TP, R, FAM>;
     using XL = typename C::XL;
-    constexpr int L = C::L, X = C::X, XP = C::XP;
+    constexpr int L = C::L, X = C::X;
     constexpr int RA = RD::RA, RB = RD::RB, RL = RD::RL, M = XL::M, SL = XL::SL, QL = XL::QL;
     constexpr bool EVEN = M % 2 == 0;  // butterfly M/2 exists
     constexpr bool c2r = FAM != XFAM_FWD;
@@ -589,11 +589,11 @@ k_xpass(XArgs a)
                 for (int kb = t; kb < C::NKB; kb += TP) prefetch_l2(S2 + (long long) kb * ks);
             }
             if (t == 0) {
-                const long long r2 = ((long long) z2 * a.Y + yy2) * XP;
-                constexpr uint32_t rb = (uint32_t) (XP * sizeof(float));
-                if (op_reads_x(op)) prefetch_l2_bulk(a.src + r2, rb);
-                if (op_reads_xp(op)) prefetch_l2_bulk(a.srcp + r2, rb);
-                if (rw) prefetch_l2_bulk(a.Wt + r2, rb);
+                const long long r2 = ((long long) z2 * a.Y + yy2) * a.X;
+                const uint32_t rb = (uint32_t) (a.X * sizeof(float));
+                if (op_reads_x(op) && a.bulk) prefetch_l2_bulk(a.src + r2, rb);
+                if (op_reads_xp(op) && a.bulk) prefetch_l2_bulk(a.srcp + r2, rb);
+                if (rw && a.bulk) prefetch_l2_bulk(a.Wt + r2, rb);
                 if (FAM == XFAM_RATIO)
                     prefetch_l2_bulk(a.g + ((long long) z2 * a.N + yy2) * a.GP, (uint32_t) (a.GP * sizeof(float)));
             }
@@ -711,7 +711,7 @@ k_xpass(XArgs a)
 
     // ---- pointwise op on x[2n], x[2n+1], n = j + r*SL
     if (row_ok) {
-        const long long rbase = ((long long) z * a.Y + yy) * XP;
+        const long long rbase = ((long long) z * a.Y + yy) * a.X;
 #pragma unroll
         for (int q = 0; q < QL; ++q) {
             const int j = t + q * TP;
