@@ -30,6 +30,7 @@
 
 #include "../../include/dwcu.h"
 #include "misc_kernels.cuh"
+#include "launch.cuh"
 #include "plans_gen.h"
 
 namespace dwcu {
@@ -549,7 +550,7 @@ struct dwcu_job {
     double *partial = nullptr;
     dwcu::JobScalars *sc = nullptr;
     float *err = nullptr;          // device error trace
-    long long *amax = nullptr;
+    dwcu::PsfPeak *peak = nullptr;
     dwcu::StatsPartial *spart = nullptr;
     dwcu::ArgmaxPartial *apart = nullptr;
     float *psf_dev = nullptr;      // staging for the PSF
@@ -559,6 +560,8 @@ struct dwcu_job {
     // iteration state
     dwcu::Iter it;
     int k_next = -1;               // iteration whose forward half runs next; -1: finished
+    bool flat0 = false;            // iteration 0's estimate is the constant x0 (flat start)
+    float x0 = 0;
     bool spectrum_ready = false;   // S holds the transform of iteration k_next's input
     int done_iters = 0;
     bool finished = false;
@@ -588,6 +591,12 @@ namespace dwcu {
 static int trace_cap(const dwcu_opts &s) { return std::max(1, std::max(s.n_iter, s.maxiter)); }
 
 // ---- pass launchers
+
+#define TRY(x)                          \
+    do {                                \
+        int rc_ = (x);                  \
+        if (rc_ != DWCU_SUCCESS) return rc_; \
+    } while (0)
 
 static int launch_lines(dwcu_job *j, const LinesPlan *p, const float2 *tw, long long n, long long line_stride,
                         long long outer_stride, long long nouter, long long ncols, int mode, float2 *data,
@@ -698,6 +707,13 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
     a.rl_clamp = 1;
     a.alpha = alpha;
     a.alpha_next = alpha_next;
+    if (op == XOP_FWD_PSF) {
+        a.pM = (int) g.pM;
+        a.pN = (int) g.pN;
+        a.pP = (int) g.pP;
+        a.peak = &j->peak->x;
+        a.scale = (float) (1.0 / ((double) g.X * (double) g.Y * (double) g.Z));
+    }
     // the OTF is the shifted PSF, not a periodic field: no margins (`field`
     // false: the transform of the OTF into another buffer)
     const bool wrap = field && S != j->K;
@@ -706,13 +722,13 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
     a.hx = (int) g.hx;
     // algorithmic traffic of this launch
     static const char *names[] = {"x_fwd_copy", "x_fwd_ones", "x_fwd_shbp", "x_ratio_shb", "x_ratio_rl",
-                                  "x_error", "x_update_shb", "x_update_rl", "x_weights", "x_store"};
+                                  "x_error", "x_update_shb", "x_update_rl", "x_weights", "x_store", "x_fwd_psf"};
     const double C = 8.0 * (double) (g.X / 2 + 1) * (double) (g.Y * g.Z);
     const double R = 4.0 * (double) g.X * (double) (g.Y * g.Z);  // algorithmic: the X used columns
     const double G = 4.0 * (double) (g.M * g.N * g.P);
-    static const double real_in[] = {1, 0, 2, 0, 0, 0, 3, 2, 0, 0};
-    static const double real_out[] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 1};
-    double bytes = (op >= XOP_RATIO_SHB ? C : 0.0) + (r2c ? C : 0.0) + (real_in[op] + real_out[op]) * R;
+    static const double real_in[] = {1, 0, 2, 0, 0, 0, 3, 2, 0, 0, 0};
+    static const double real_out[] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 1, 0};
+    double bytes = (x_family(op) != XFAM_FWD ? C : 0.0) + (r2c ? C : 0.0) + (real_in[op] + real_out[op]) * R;
     if (op == XOP_UPDATE_SHB && !j->W) bytes -= R;
     if (op == XOP_UPDATE_RL && !j->W) bytes -= R;
     if (op == XOP_RATIO_SHB || op == XOP_RATIO_RL || op == XOP_ERROR_ONLY) {
@@ -729,11 +745,20 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
     CHECK_LAUNCH();
     if (r2c && wrap && (g.wy || g.wz)) {
         // periodic y/z: margin rows of the new spectrum copy the rows they wrap to
-        const long long segs = g.Z * g.NKB * g.Y;
-        const int blocks = (int) std::min<long long>(148 * 16, (segs + 255) / 256);
-        k_wrap_rows<<<blocks, 256, 0, j->stream>>>(S, (int) g.Y, (int) g.Z, (int) g.NKB, (int) g.wN, (int) g.hy,
-                                                   g.wy ? 1 : 0, (int) g.wP, (int) g.hz, g.wz ? 1 : 0);
-        CHECK_LAUNCH();
+        WrapArgs w{S, (int) g.Y, (int) g.Z, (int) g.NKB, (int) g.wN, (int) g.hy, g.wy ? 1 : 0,
+                   (int) g.wP, (int) g.hz, g.wz ? 1 : 0, 0, 0, 0};
+        auto rows = [&](long long y0, long long ny, long long z0, long long nz) -> int {
+            if (ny < 1 || nz < 1) return DWCU_SUCCESS;
+            w.y0 = (int) y0;
+            w.ny = (int) ny;
+            w.z0 = (int) z0;
+            launch_dep(k_wrap_rows, dim3((unsigned) ((2 * ny + 63) / 64), (unsigned) g.NKB, (unsigned) nz), dim3(64), 0,
+                       j->stream, w);
+            CHECK_LAUNCH();
+            return DWCU_SUCCESS;
+        };
+        if (g.wy) TRY(rows(g.wN, g.Y - g.wN, 0, g.wz ? g.wP : g.Z));
+        if (g.wz) TRY(rows(0, g.Y, g.wP, g.Z - g.wP));
     }
     return DWCU_SUCCESS;
 }
@@ -741,16 +766,11 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
 static int err_final(dwcu_job *j, int k, long long tiles)
 {
     const Geometry &g = j->g;
-    k_err_final<<<1, kRedThreads, 0, j->stream>>>(j->partial, (int) tiles, (double) (g.M * g.N * g.P), j->err + k);
+    launch_dep(k_err_final, dim3(1), dim3(kErrThreads), 0, j->stream,
+               ErrArgs{j->partial, (int) tiles, (double) (g.M * g.N * g.P), j->err + k});
     CHECK_LAUNCH();
     return DWCU_SUCCESS;
 }
-
-#define TRY(x)                          \
-    do {                                \
-        int rc_ = (x);                  \
-        if (rc_ != DWCU_SUCCESS) return rc_; \
-    } while (0)
 
 // method_shb.c:328-330: alpha = clamp((k - 1)/(k + 2), 0, alphamax)
 static double shb_alpha(int k, float alphamax)
@@ -823,13 +843,20 @@ static int iter_forward(dwcu_job *j, int k, bool ratio)
 {
     const Geometry &g = j->g;
     const bool shb = (j->s.method == DWCU_METHOD_SHB);
-    TRY(conv_forward(j));
+    if (k == 0 && j->flat0) {
+        // a constant needs no transforms (iter_input left S alone)
+        launch_dep(k_flat_rows, dim3((unsigned) ((2 * g.Y + 127) / 128), (unsigned) g.NKB, (unsigned) g.P), dim3(128), 0,
+                   j->stream, FlatArgs{j->S, j->sc, (int) g.Y, (int) g.NKB, shb ? 1 : 0});
+        CHECK_LAUNCH();
+    } else {
+        TRY(conv_forward(j));
+    }
     int op = ratio ? (shb ? XOP_RATIO_SHB : XOP_RATIO_RL) : XOP_ERROR_ONLY;
     const long long ytiles = (g.Y + g.xp->R - 1) / g.xp->R;
     // planes z >= P are read later by RL, and by a periodic z (its margins)
     const long long tiles = (op == XOP_RATIO_RL || g.wz) ? j->nxb : g.P * ytiles;
     TRY(pass_x(j, op, ratio ? 1 : 0, j->S, nullptr, nullptr, nullptr, 0, 0, tiles));
-    TRY(err_final(j, k, tiles));
+    TRY(err_final(j, k, g.P * ytiles));  // the tiles of planes z >= P add nothing
     return DWCU_SUCCESS;
 }
 
@@ -852,6 +879,7 @@ static int iter_backward(dwcu_job *j, int k, bool next)
 // transform of iteration k's input (p_k for SHB, x_k for RL) into S
 static int iter_input(dwcu_job *j, int k)
 {
+    if (k == 0 && j->flat0) return DWCU_SUCCESS;  // iter_forward needs no transform of it
     if (j->s.method == DWCU_METHOD_SHB)
         return pass_x(j, XOP_FWD_SHBP, 1, j->S, j->xa, j->xb, nullptr, shb_alpha(k, j->s.alphamax), 0);
     return pass_x(j, XOP_FWD_COPY, 1, j->S, j->xa, nullptr, nullptr, 0, 0);
@@ -903,7 +931,7 @@ static int alloc_job(dwcu_job *j)
     size_t o_part = take(sizeof(double) * (size_t) j->nxb);
     size_t o_sc = take(sizeof(JobScalars));
     size_t o_err = take(sizeof(float) * (size_t) trace_cap(j->s));
-    size_t o_amax = take(sizeof(long long));
+    size_t o_peak = take(sizeof(PsfPeak));
     size_t o_sp = take(sizeof(StatsPartial) * (size_t) j->n_spart);
     size_t o_ap = take(sizeof(ArgmaxPartial) * (size_t) j->n_apart);
     size_t o_psf = take(sizeof(float) * (size_t) npsf);
@@ -927,7 +955,7 @@ static int alloc_job(dwcu_job *j)
     j->partial = (double *) (b + o_part);
     j->sc = (JobScalars *) (b + o_sc);
     j->err = (float *) (b + o_err);
-    j->amax = (long long *) (b + o_amax);
+    j->peak = (PsfPeak *) (b + o_peak);
     j->spart = (StatsPartial *) (b + o_sp);
     j->apart = (ArgmaxPartial *) (b + o_ap);
     j->psf_dev = (float *) (b + o_psf);
@@ -1267,14 +1295,14 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
     const int nab = (int) ((npsf + per - 1) / per);
     k_argmax_partial<<<nab, kRedThreads, 0, st>>>(j->psf_dev, npsf, per, j->apart, &j->sc->flags);
     CHECK_LAUNCH();
-    k_argmax_final<<<1, 32, 0, st>>>(j->apart, nab, j->amax);
+    k_argmax_final<<<1, kRedThreads, 0, st>>>(j->apart, nab, (int) g.pM, (int) g.pN, j->peak, j->sc);
     CHECK_LAUNCH();
     if (g.wx || g.wy || g.wz) {
         // the periodic margins assume the PSF maximum within h of both ends
-        long long am = 0;
-        CU(cudaMemcpyAsync(&am, j->amax, sizeof am, cudaMemcpyDeviceToHost, st));
+        PsfPeak pk{};
+        CU(cudaMemcpyAsync(&pk, j->peak, sizeof pk, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
-        const long long ax = am % g.pM, ay = (am / g.pM) % g.pN, az = am / (g.pM * g.pN);
+        const long long ax = pk.x, ay = pk.y, az = pk.z;
         auto off = [](long long a, long long p) { return std::max(a, p - 1 - a); };
         if ((g.wx && off(ax, g.pM) > g.hx) || (g.wy && off(ay, g.pN) > g.hy) || (g.wz && off(az, g.pP) > g.hz))
             return fail(DWCU_ERROR_UNSUPPORTED,
@@ -1282,23 +1310,36 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
                         "its centre (maximum at %lld, %lld, %lld of %lld x %lld x %lld)",
                         j->s.border_quality, ax, ay, az, g.pM, g.pN, g.pP);
     }
+    // (Columns past X/2 of the blocked layout are transformed along and read
+    // by nothing, so the spectra need no clearing.)
     const size_t R = sizeof(float) * (size_t) g.real_elems();
-    CU(cudaMemsetAsync(j->S, 0, sizeof(float2) * (size_t) g.spec_elems(), st));
-    CU(cudaMemsetAsync(j->K, 0, sizeof(float2) * (size_t) g.spec_elems(), st));
-    CU(cudaMemsetAsync(j->xb, 0, R, st));
-    const float scale = (float) (1.0 / ((double) g.X * (double) g.Y * (double) g.Z));
-    k_psf_embed<<<(int) std::min<long long>(4096, (npsf + 255) / 256), 256, 0, st>>>(
-        j->psf_dev, (int) g.pM, (int) g.pN, (int) g.pP, j->amax, j->xb, (int) g.X, (int) g.Y, (int) g.Z,
-        (int) g.XP, scale);
-    CHECK_LAUNCH();
-    TRY(pass_x(j, XOP_FWD_COPY, 1, j->K, j->xb, nullptr, nullptr, 0, 0));
+    if (g.pM <= g.X && g.pN <= g.Y && g.pP <= g.Z) {
+        TRY(pass_x(j, XOP_FWD_PSF, 1, j->K, j->psf_dev, nullptr, nullptr, 0, 0));
+    } else {
+        const float scale = (float) (1.0 / ((double) g.X * (double) g.Y * (double) g.Z));
+        CU(cudaMemsetAsync(j->xb, 0, R, st));
+        k_psf_embed<<<(int) std::min<long long>(4096, (npsf + 255) / 256), 256, 0, st>>>(
+            j->psf_dev, (int) g.pM, (int) g.pN, (int) g.pP, j->peak, j->xb, (int) g.X, (int) g.Y, (int) g.Z,
+            (int) g.XP, scale);
+        CHECK_LAUNCH();
+        TRY(pass_x(j, XOP_FWD_COPY, 1, j->K, j->xb, nullptr, nullptr, 0, 0));
+    }
     TRY(pass_y(j, LINES_FWD, j->K));
     TRY(pass_z(j, LINES_FWD, j->K));
 
     // Bertero weights: W = 1/P1 where P1 = K^T 1_image > 0.01 (method_shb.c:216-235)
     if (j->W) {
-        TRY(pass_x(j, XOP_FWD_ONES, 1, j->S, nullptr, nullptr, nullptr, 0, 0));
-        TRY(conv(j, 1));
+        if (g.wz || one_plane(g)) {
+            TRY(pass_x(j, XOP_FWD_ONES, 1, j->S, nullptr, nullptr, nullptr, 0, 0));
+            TRY(conv(j, 1));
+        } else {
+            // the planes z >= P are zero: neither made nor read
+            const long long ytiles = (g.Y + g.xp->R - 1) / g.xp->R;
+            TRY(pass_x(j, XOP_FWD_ONES, 1, j->S, nullptr, nullptr, nullptr, 0, 0, g.P * ytiles));
+            TRY(pass_y(j, LINES_FWD, j->S, g.P));
+            TRY(pass_z(j, LINES_CONV_CONJ, j->S, g.P, g.Z));
+            TRY(pass_y(j, LINES_INV, j->S));
+        }
         TRY(pass_x(j, XOP_WEIGHTS, 0, j->S, nullptr, nullptr, j->W, 0, 0));
     }
 
@@ -1319,7 +1360,7 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
     const long long nv = g.real_elems();
     const int fb = (int) std::min<long long>(148 * 16, (nv + 255) / 256);
     if (j->s.start_condition == DWCU_START_FLAT) {
-        k_fill_scalar<<<fb, 256, 0, st>>>(j->xa, nv, j->sc);
+        k_fill_scalar<<<fb, 256, 0, st>>>(j->xa, j->s.method == DWCU_METHOD_SHB ? j->xb : nullptr, nv, j->sc);
         CHECK_LAUNCH();
     } else if (j->s.start_condition == DWCU_START_LP) {
         // method_shb.c:278-285, method_rl.c:290-297: the image smoothed by
@@ -1358,7 +1399,9 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
                                           (int) g.Y);
         CHECK_LAUNCH();
     }
-    if (j->s.method == DWCU_METHOD_SHB) CU(cudaMemcpyAsync(j->xb, j->xa, R, cudaMemcpyDeviceToDevice, st));
+    j->flat0 = j->s.start_condition == DWCU_START_FLAT;
+    if (j->s.method == DWCU_METHOD_SHB && !j->flat0)
+        CU(cudaMemcpyAsync(j->xb, j->xa, R, cudaMemcpyDeviceToDevice, st));
 
     // input flags (non-finite values) are checked once, here
     JobScalars hs;
@@ -1367,6 +1410,7 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
     if (hs.flags & 1) return fail(DWCU_ERROR_INPUT, "the image contains non-finite values");
     if (hs.flags & 2) return fail(DWCU_ERROR_INPUT, "the PSF contains non-finite values");
     if (j->s.bg_auto) j->s.bg = hs.bg;
+    j->x0 = hs.x0;
     j->it.init(j->s);
     j->k_next = j->it.next();
     j->finished = (j->k_next < 0);
@@ -1430,10 +1474,10 @@ static int job_step_impl(dwcu_job *j, int nmax, int *remaining)
                 char key[512];
                 const Geometry &gg = j->g;
                 snprintf(key, sizeof key,
-                         "%lld %lld %lld %lld %lld %lld %lld %lld %lld|%d %d %d %d %d %d %d %a|%d %d %d %p %p|%p %p %p %p",
+                         "%lld %lld %lld %lld %lld %lld %lld %lld %lld|%d %d %d %d %d %d %d %a|%d %d %d %d %p %p|%p %p %p %p",
                          gg.M, gg.N, gg.P, gg.pM, gg.pN, gg.pP, gg.X, gg.Y, gg.Z, j->s.method, j->it.niter,
                          j->s.maxiter, k, j->s.metric, j->s.positivity, j->s.border_quality, (double) j->s.alphamax,
-                         (int) j->spectrum_ready, (int) (j->W != nullptr), (int) prof, (void *) j->xa, (void *) j->xb,
+                         (int) j->spectrum_ready, (int) j->flat0, (int) (j->W != nullptr), (int) prof, (void *) j->xa, (void *) j->xb,
                          (const void *) gg.xp, (const void *) gg.yp, (const void *) gg.zp, (const void *) gg.ytp);
                 const std::string skey(key);
                 cudaGraphExec_t ex = nullptr;
@@ -2091,6 +2135,12 @@ int dwcu_job_restore(dwcu_job *j, const float *x, const float *x_prev, const flo
     j->it.lasterror = st->lasterror;
     j->spectrum_ready = false;
     j->spec = -1;
+    if (j->flat0) {
+        // the shortcut for a constant first estimate holds for this one only
+        // if it is still that constant
+        const long long n = st->volume_elems;
+        for (long long i = 0; i < n && j->flat0; ++i) j->flat0 = x[i] == j->x0 && (!shb || x_prev[i] == j->x0);
+    }
     return DWCU_SUCCESS;
 }
 

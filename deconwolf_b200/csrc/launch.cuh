@@ -45,6 +45,26 @@ inline int persistent_grid(KernelOnce &ko, K kernel, int threads, size_t smem, i
     return ntiles < g ? ntiles : g;
 }
 
+// A launch that may overlap the end of the kernel before it on the stream
+// (the kernel calls dep_wait, tma.cuh).  It hides the launch latency between
+// passes: 48 x 40 x 10, SHB 10 (102 launches) 408 -> 370 us, 317 x 241 x 33
+// periodic 2372 -> 2309, 2048 x 2048 x 60 unchanged.
+template <class A>
+inline void launch_dep(void (*kernel)(A), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A &a)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 template <class RD, int T>
 void launch_lines_t(const LinesArgs &a, int nblocks, cudaStream_t st)
 {
@@ -54,10 +74,10 @@ void launch_lines_t(const LinesArgs &a, int nblocks, cudaStream_t st)
     const size_t smem = a.mode >= LINES_CONV ? C::SMEM_BYTES : C::SMEM_FFT;
     if (a.planes || a.packed) {
         ensure_smem(kp, k_lines<RD, T, true>, C::SMEM_BYTES);
-        k_lines<RD, T, true><<<nblocks, dim3(T, tpl), smem, st>>>(a);
+        launch_dep(k_lines<RD, T, true>, dim3(nblocks), dim3(T, tpl), smem, st, a);
     } else {
         ensure_smem(ko, k_lines<RD, T>, C::SMEM_BYTES);
-        k_lines<RD, T><<<nblocks, dim3(T, tpl), smem, st>>>(a);
+        launch_dep(k_lines<RD, T>, dim3(nblocks), dim3(T, tpl), smem, st, a);
     }
 }
 
@@ -68,7 +88,7 @@ void launch_y_dir(const YArgs &a, cudaStream_t st)
     using C = YCfg<RD>;
     ensure_smem(ko, k_ypass<RD, DIR>, C::SMEM_BYTES);
     const int grid = persistent_grid(ko, k_ypass<RD, DIR>, C::THREADS, C::SMEM_BYTES, a.ntiles);
-    k_ypass<RD, DIR><<<grid, dim3(C::TX, RD::TPL), C::SMEM_BYTES, st>>>(a);
+    launch_dep(k_ypass<RD, DIR>, dim3(grid), dim3(C::TX, RD::TPL), C::SMEM_BYTES, st, a);
 }
 
 template <class RD>
@@ -86,7 +106,7 @@ void launch_yconv_t(const YArgs &a, cudaStream_t st)
     static KernelOnce ko;
     using C = YConvCfg<RD>;
     ensure_smem(ko, k_yconv<RD>, C::SMEM_BYTES);
-    k_yconv<RD><<<a.ntiles, dim3(KB, C::TPL), C::SMEM_BYTES, st>>>(a);
+    launch_dep(k_yconv<RD>, dim3(a.ntiles), dim3(KB, C::TPL), C::SMEM_BYTES, st, a);
 }
 
 }  // namespace dwcu

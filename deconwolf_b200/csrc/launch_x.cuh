@@ -15,7 +15,7 @@ void launch_x_fam(const XArgs &a, cudaStream_t st)
     const int planes = a.ntiles / ((a.Y + R - 1) / R);
     if (planes < 1) return;
     ensure_smem(ko, k_xpass<RD, TP, RF, FAM>, C::SMEM_BYTES);
-    k_xpass<RD, TP, RF, FAM><<<dim3((a.Y + RF - 1) / RF, planes), dim3(TP, RF), C::SMEM_BYTES, st>>>(a);
+    launch_dep(k_xpass<RD, TP, RF, FAM>, dim3((a.Y + RF - 1) / RF, planes), dim3(TP, RF), C::SMEM_BYTES, st, a);
 }
 
 // Rows that fill whole warps by themselves run one per CTA, except in the

@@ -107,6 +107,12 @@ k_stats_final(const StatsPartial *__restrict__ part, int nb, JobScalars *sc, int
 struct ArgmaxPartial {
     float v;
     long long i;
+    double sum;
+};
+// where the PSF's first maximum lies: linear index, x, y, z
+struct PsfPeak {
+    long long i;
+    int x, y, z;
 };
 
 // first maximum (lowest linear index), fim_argmax_max fim.c:269-332
@@ -123,8 +129,10 @@ k_argmax_partial(const float *__restrict__ a, long long n, long long per_block, 
 {
     __shared__ float sv[kRedThreads];
     __shared__ long long si[kRedThreads];
+    __shared__ double ss[kRedThreads];
     float v = -INFINITY;
     long long idx = LLONG_MAX;
+    double sum = 0.0;
     const long long b0 = (long long) blockIdx.x * per_block;
     const long long b1 = min(n, b0 + per_block);
     int nf = 0;
@@ -132,10 +140,12 @@ k_argmax_partial(const float *__restrict__ a, long long n, long long per_block, 
         float x = a[k];
         if (!isfinite(x)) nf = 1;
         amax_merge(v, idx, x, k);
+        sum += (double) x;
     }
     if (nf) atomicOr(flags, 2);
     sv[threadIdx.x] = v;
     si[threadIdx.x] = idx;
+    ss[threadIdx.x] = sum;
     __syncthreads();
     for (int o = kRedThreads / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) {
@@ -146,33 +156,61 @@ k_argmax_partial(const float *__restrict__ a, long long n, long long per_block, 
             amax_merge(v1, i1, v2, i2);
             sv[threadIdx.x] = v1;
             si[threadIdx.x] = i1;
+            ss[threadIdx.x] += ss[threadIdx.x + o];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = ArgmaxPartial{sv[0], si[0]};
+    if (threadIdx.x == 0) part[blockIdx.x] = ArgmaxPartial{sv[0], si[0], ss[0]};
 }
 
-__global__ void k_argmax_final(const ArgmaxPartial *part, int nb, long long *out)
+// One block of kRedThreads: the peak and the PSF's sum (in double, fixed order).
+__global__ void __launch_bounds__(kRedThreads)
+k_argmax_final(const ArgmaxPartial *part, int nb, int pM, int pN, PsfPeak *out, JobScalars *sc)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ float sv[kRedThreads];
+    __shared__ long long si[kRedThreads];
+    __shared__ double ss[kRedThreads];
+    const int t = threadIdx.x;
     float v = -INFINITY;
     long long i = LLONG_MAX;
-    for (int b = 0; b < nb; ++b) amax_merge(v, i, part[b].v, part[b].i);
-    *out = i;
+    double sum = 0.0;
+    for (int b = t; b < nb; b += kRedThreads) {
+        amax_merge(v, i, part[b].v, part[b].i);
+        sum += part[b].sum;
+    }
+    sv[t] = v;
+    si[t] = i;
+    ss[t] = sum;
+    __syncthreads();
+    for (int o = kRedThreads / 2; o > 0; o >>= 1) {
+        if (t < o) {
+            float v1 = sv[t];
+            long long i1 = si[t];
+            amax_merge(v1, i1, sv[t + o], si[t + o]);
+            sv[t] = v1;
+            si[t] = i1;
+            ss[t] += ss[t + o];
+        }
+        __syncthreads();
+    }
+    if (t == 0) {
+        const long long am = si[0], r = am / pM;
+        *out = PsfPeak{am, (int) (am % pM), (int) (r % pN), (int) (r / pN)};
+        sc->psfsum = ss[0];
+    }
 }
 
 // Place the PSF into a zeroed X x Y x Z volume so that its first maximum
 // lands at the origin (fim_insert fim.c:585-623 followed by fim_circshift
 // fim.c:982-1057 by minus the argmax), scaled by `scale` (the inverse
-// transform normalisation 1/(X*Y*Z) is folded into the OTF here).
-__global__ void k_psf_embed(const float *__restrict__ psf, int pM, int pN, int pP, const long long *amax,
+// transform normalisation 1/(X*Y*Z) is folded into the OTF here).  For PSFs
+// larger than the job along an axis; others are read by the x pass as they
+// lie (XOP_FWD_PSF).
+__global__ void k_psf_embed(const float *__restrict__ psf, int pM, int pN, int pP, const PsfPeak *peak,
                             float *__restrict__ dst, int X, int Y, int Z, int XP, float scale)
 {
     const long long n = (long long) pM * pN * pP;
-    const long long am = *amax;
-    const int ac = (int) (am / ((long long) pM * pN));
-    const int ab = (int) ((am - (long long) ac * pM * pN) / pM);
-    const int aa = (int) (am - (long long) ac * pM * pN - (long long) ab * pM);
+    const int aa = peak->x, ab = peak->y, ac = peak->z;
     for (long long k = blockIdx.x * (long long) blockDim.x + threadIdx.x; k < n;
          k += (long long) gridDim.x * blockDim.x) {
         const int c = (int) (k / ((long long) pM * pN));
@@ -185,12 +223,38 @@ __global__ void k_psf_embed(const float *__restrict__ psf, int pM, int pN, int p
     }
 }
 
-__global__ void k_fill_scalar(float *__restrict__ x, long long n, const JobScalars *sc)
+// the flat start: x_0, and x_{-1} = x_0 where there is one (n: a multiple of 4)
+__global__ void k_fill_scalar(float *__restrict__ x, float *__restrict__ xp, long long n, const JobScalars *sc)
 {
     const float v = sc->x0;
-    for (long long k = blockIdx.x * (long long) blockDim.x + threadIdx.x; k < n;
-         k += (long long) gridDim.x * blockDim.x)
-        x[k] = v;
+    const float4 v4 = make_float4(v, v, v, v);
+    for (long long k = blockIdx.x * (long long) blockDim.x + threadIdx.x; k < n / 4;
+         k += (long long) gridDim.x * blockDim.x) {
+        reinterpret_cast<float4 *>(x)[k] = v4;
+        if (xp) reinterpret_cast<float4 *>(xp)[k] = v4;
+    }
+}
+
+// The first forward convolution of a flat start, as the inverse y pass would
+// leave it on the image planes: K p of a constant p is the constant p times
+// the PSF's sum (in double, rounded once), whose rows have a spectrum at
+// kx = 0 only.  `clamp`: SHB's p_0 = max(x_0, bg).  Block z: plane blockIdx.z.
+struct FlatArgs {
+    float2 *S;
+    const JobScalars *sc;
+    int Y, nkb, clamp;
+};
+__global__ void k_flat_rows(FlatArgs a)
+{
+    dep_wait();
+    const int h = blockIdx.x * blockDim.x + threadIdx.x;  // half of a row's kx block: 16 bytes
+    if (h >= 2 * a.Y) return;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (blockIdx.y == 0 && h % 2 == 0) {
+        const float x0 = a.sc->x0, bg = a.sc->bg;
+        v.x = (float) ((double) (a.clamp && x0 < bg ? bg : x0) * a.sc->psfsum);
+    }
+    reinterpret_cast<float4 *>(a.S + ((long long) blockIdx.z * a.nkb + blockIdx.y) * a.Y * KB)[h] = v;
 }
 
 // image into the corner of a zeroed real volume (start_condition IDENTITY)
@@ -263,33 +327,27 @@ __global__ void k_gsmooth_axis(const float *__restrict__ in, float *__restrict__
 // Periodic y and/or z (bq 0/1 axes transformed at a larger length): after a
 // forward x pass, every spectrum row (y, z) outside [0, wN) x [0, wP) takes
 // a copy of the row it wraps to -- [w, w+h) from [0, h), [len-h, len) from
-// [w-h, w) -- and the rows in between are cleared.  One thread per 4-wide
-// kx block of a row.
-__global__ void k_wrap_rows(float2 *__restrict__ S, int Y, int Z, int nkb, int wN, int hy, int wrapy, int wP, int hz,
-                            int wrapz)
+// [w-h, w) -- and the rows in between are cleared.  A launch covers the rows
+// [y0, y0+ny) of the planes z0 + blockIdx.z, margins only; two threads per
+// 4-wide kx block of a row.
+struct WrapArgs {
+    float2 *S;
+    int Y, Z, nkb, wN, hy, wrapy, wP, hz, wrapz;
+    int y0, ny, z0;
+};
+__global__ void k_wrap_rows(WrapArgs a)
 {
-    const long long n = (long long) Z * nkb * Y;
-    for (long long e = blockIdx.x * (long long) blockDim.x + threadIdx.x; e < n;
-         e += (long long) gridDim.x * blockDim.x) {
-        const int y = (int) (e % Y);
-        const long long zk = e / Y;
-        const int kb = (int) (zk % nkb);
-        const int z = (int) (zk / nkb);
-        const bool yin = !wrapy || y < wN, zin = !wrapz || z < wP;
-        if (yin && zin) continue;
-        auto src = [](int v, int w, int h, int len) { return v < w ? v : v < w + h ? v - w : v >= len - h ? v - len + w : -1; };
-        const int ys = wrapy ? src(y, wN, hy, Y) : y;
-        const int zs = wrapz ? src(z, wP, hz, Z) : z;
-        float2 *dst = S + (((long long) z * nkb + kb) * Y + y) * KB;
-        if (ys < 0 || zs < 0) {
-#pragma unroll
-            for (int i = 0; i < KB; ++i) dst[i] = make_float2(0.f, 0.f);
-        } else {
-            const float2 *from = S + (((long long) zs * nkb + kb) * Y + ys) * KB;
-#pragma unroll
-            for (int i = 0; i < KB; ++i) dst[i] = from[i];
-        }
-    }
+    dep_wait();
+    const int h = blockIdx.x * blockDim.x + threadIdx.x;  // half of a row's kx block: 16 bytes
+    if (h >= 2 * a.ny) return;
+    const int y = a.y0 + h / 2, kb = blockIdx.y, z = a.z0 + (int) blockIdx.z;
+    auto src = [](int v, int w, int h, int len) { return v < w ? v : v < w + h ? v - w : v >= len - h ? v - len + w : -1; };
+    const int ys = a.wrapy ? src(y, a.wN, a.hy, a.Y) : y;
+    const int zs = a.wrapz ? src(z, a.wP, a.hz, a.Z) : z;
+    auto at = [&](int zz, int yy) {
+        return reinterpret_cast<float4 *>(a.S + (((long long) zz * a.nkb + kb) * a.Y + yy) * KB) + h % 2;
+    };
+    *at(z, y) = ys < 0 || zs < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *at(zs, ys);
 }
 
 // fim_subregion (fim.c:695-718): the image-sized corner of a job volume
@@ -307,19 +365,35 @@ __global__ void k_crop(const float *__restrict__ x, int X, int Y, int M, int N, 
 
 // finish one iteration's error: mean over the image of the x-pass partials
 // (get_fIdiv dw.c:1492-1524 / get_fMSE dw.c:1461-1490)
-__global__ void __launch_bounds__(kRedThreads)
-k_err_final(const double *__restrict__ part, int nb, double count, float *err_out)
+constexpr int kErrThreads = 1024;
+
+// the sum of nb partials by one block of kErrThreads, in a fixed order
+// (valid on thread 0)
+__device__ __forceinline__ double err_block_sum(const double *part, int nb)
 {
-    __shared__ double s[kRedThreads];
+    __shared__ double s[kErrThreads];
     double v = 0.0;
-    for (int i = threadIdx.x; i < nb; i += kRedThreads) v += part[i];
+    for (int i = threadIdx.x; i < nb; i += kErrThreads) v += part[i];
     s[threadIdx.x] = v;
     __syncthreads();
-    for (int o = kRedThreads / 2; o > 0; o >>= 1) {
+    for (int o = kErrThreads / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *err_out = (float) (s[0] / count);
+    return s[0];
+}
+
+struct ErrArgs {
+    const double *part;
+    int nb;
+    double count;
+    float *out;
+};
+__global__ void __launch_bounds__(kErrThreads) k_err_final(ErrArgs a)
+{
+    dep_wait();
+    const double v = err_block_sum(a.part, a.nb);
+    if (threadIdx.x == 0) *a.out = (float) (v / a.count);
 }
 
 }  // namespace dwcu

@@ -295,6 +295,7 @@ k_lines(LinesArgs a)
     using Cfg = LinesCfg<RD, T>;
     float2 *sotf = sm + Cfg::XCH_F2;  // OTF tile [n][col] (convolve modes)
     const int col0 = tile * T;
+    dep_wait();
     if (mode >= LINES_CONV && (T % 2) == 0) {
         // the tile's OTF columns arrive while the forward transform runs:
         // 16-byte pieces (two columns) of each of the N rows
@@ -323,6 +324,7 @@ k_lines(LinesArgs a)
         line_fft<RD, -1, 1>(v, o, t, a.tw, smem);
     constexpr int SL = N / RD::RL;
     if (mode == LINES_FWD || mode == LINES_INV) {
+        dep_start_next();
         if (t < SL && valid_out) {
 #pragma unroll
             for (int r = 0; r < RD::RL; ++r)
@@ -353,6 +355,7 @@ k_lines(LinesArgs a)
     float2 q[1][RV::RL];
     line_fft<RV, +1, 1>(o, q, t, a.tw, smem);
     constexpr int SQ = N / RV::RL;
+    dep_start_next();
     if (t < SQ && valid) {
 #pragma unroll
         for (int r = 0; r < RV::RL; ++r)
@@ -414,6 +417,7 @@ k_ypass(YArgs a)
                                        t < N / (RD::THREE ? RD::RC : 1) ? t : 0, a.tw)
                                  : make_float2(1.f, 0.f);
     int tile = blockIdx.x;
+    dep_wait();
     if (tid == 0 && tile < a.ntiles) {
         mbar_arrive_expect_tx(&bars[0], C::TILE_BYTES);
         tma_load_1d(bufs, a.data + (size_t) tile * N * KB, C::TILE_BYTES, &bars[0]);
@@ -424,6 +428,7 @@ k_ypass(YArgs a)
         fence_proxy_async();  // this thread's accesses to the other buffer precede the next bulk copy into it
         __syncthreads();      // the other buffer is no longer read
         const int next = tile + gridDim.x;
+        if (next >= a.ntiles) dep_start_next();
         if (tid == 0 && next < a.ntiles) {
             fence_proxy_async();
             mbar_arrive_expect_tx(&bars[b ^ 1], C::TILE_BYTES);
@@ -495,6 +500,7 @@ k_yconv(YArgs a)
     float2 *A = reinterpret_cast<float2 *>(ysm + 64), *B = A + C::BUF_F2;
     const int l = threadIdx.x, t = threadIdx.y;
     float2 *tile = a.data + (size_t) blockIdx.x * N * KB;
+    dep_wait();
     if (t == 0 && l == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();

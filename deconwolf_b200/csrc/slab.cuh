@@ -71,14 +71,11 @@ static void slab_layout(long long Z, long long P, long long cols, int n, int p, 
 
 // k_psf_embed restricted to one part's planes: the PSF voxel that lands on
 // plane z goes to local plane z / n when z % n == p
-__global__ void k_slab_psf_embed(const float *__restrict__ psf, int pM, int pN, int pP, const long long *amax,
+__global__ void k_slab_psf_embed(const float *__restrict__ psf, int pM, int pN, int pP, const PsfPeak *peak,
                                  float *__restrict__ dst, int X, int Y, int Z, int XP, float scale, int n, int p)
 {
     const long long cnt = (long long) pM * pN * pP;
-    const long long am = *amax;
-    const int ac = (int) (am / ((long long) pM * pN));
-    const int ab = (int) ((am - (long long) ac * pM * pN) / pM);
-    const int aa = (int) (am - (long long) ac * pM * pN - (long long) ab * pM);
+    const int aa = peak->x, ab = peak->y, ac = peak->z;
     for (long long k = blockIdx.x * (long long) blockDim.x + threadIdx.x; k < cnt;
          k += (long long) gridDim.x * blockDim.x) {
         const int c = (int) (k / ((long long) pM * pN));
@@ -93,18 +90,10 @@ __global__ void k_slab_psf_embed(const float *__restrict__ psf, int pM, int pN, 
 }
 
 // the sum of a part's tile partials, in the fixed order of k_err_final
-__global__ void __launch_bounds__(kRedThreads) k_slab_err_sum(const double *__restrict__ part, int nb, double *out)
+__global__ void __launch_bounds__(kErrThreads) k_slab_err_sum(const double *__restrict__ part, int nb, double *out)
 {
-    __shared__ double s[kRedThreads];
-    double v = 0.0;
-    for (int i = threadIdx.x; i < nb; i += kRedThreads) v += part[i];
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = kRedThreads / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = s[0];
+    const double v = err_block_sum(part, nb);
+    if (threadIdx.x == 0) *out = v;
 }
 
 // the parts' sums in part order: the iteration's error value
@@ -519,13 +508,14 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
         const int nab = (int) ((npsf + per - 1) / per);
         k_argmax_partial<<<nab, kRedThreads, 0, st>>>(j->psf_dev, npsf, per, j->apart, &j->sc->flags);
         CHECK_LAUNCH();
-        k_argmax_final<<<1, 32, 0, st>>>(j->apart, nab, j->amax);
+        k_argmax_final<<<1, kRedThreads, 0, st>>>(j->apart, nab, (int) g.pM, (int) g.pN, j->peak, j->sc);
         CHECK_LAUNCH();
     }
     // the parts' statistics, combined in part order (k_stats_final's
     // formulas), go back to every part
     double sumg = 0.0;
     float gmin = INFINITY, gmax = 0.f;
+    double psfsum = 0.0;  // the same on every part: each has the whole PSF
     int flags = 0;
     for (auto &pt : sl->parts) {
         if (!pt.j) continue;
@@ -534,6 +524,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
         CU(cudaMemcpyAsync(&hs, pt.j->sc, sizeof hs, cudaMemcpyDeviceToHost, pt.stream));
         CU(cudaStreamSynchronize(pt.stream));
         flags |= hs.flags;
+        psfsum = hs.psfsum;
         if (pt.pl > 0) {
             sumg += hs.sumg;
             gmin = std::fmin(gmin, hs.gmin);
@@ -565,11 +556,11 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
     if (flags & 2) return fail(DWCU_ERROR_INPUT, "the PSF contains non-finite values");
     if (g.wx || g.wy) {
         // the periodic margins assume the PSF maximum within h of both ends (as job_setup)
-        long long am = 0;
+        PsfPeak pk{};
         SlabPart &p0 = sl->lead();
         CU(cudaSetDevice(p0.device));
-        CU(cudaMemcpy(&am, p0.j->amax, sizeof am, cudaMemcpyDeviceToHost));
-        const long long ax = am % g.pM, ay = (am / g.pM) % g.pN;
+        CU(cudaMemcpy(&pk, p0.j->peak, sizeof pk, cudaMemcpyDeviceToHost));
+        const long long ax = pk.x, ay = pk.y;
         auto off = [](long long a, long long p) { return std::max(a, p - 1 - a); };
         if ((g.wx && off(ax, g.pM) > g.hx) || (g.wy && off(ay, g.pN) > g.hy))
             return fail(DWCU_ERROR_UNSUPPORTED,
@@ -580,6 +571,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
     JobScalars all{};
     all.gmin = gmin;
     all.gmax = gmax;
+    all.psfsum = psfsum;
     all.sumg = sumg;
     all.bg = sl->s.bg_auto ? (gmin < 1e-2f ? 1e-2f : gmin) : sl->s.bg;
     all.x0 = (float) sumg / (float) wmnp;
@@ -598,7 +590,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
         // the OTF: PSF planes of this part, x and y transforms here
         CU(cudaMemsetAsync(j->xb, 0, sizeof(float) * (size_t) j->g.real_elems(), st));
         k_slab_psf_embed<<<(int) std::min<long long>(4096, (npsf + 255) / 256), 256, 0, st>>>(
-            j->psf_dev, (int) g.pM, (int) g.pN, (int) g.pP, j->amax, j->xb, (int) g.X, (int) g.Y, (int) g.Z,
+            j->psf_dev, (int) g.pM, (int) g.pN, (int) g.pP, j->peak, j->xb, (int) g.X, (int) g.Y, (int) g.Z,
             (int) g.XP, scale, n, p);
         CHECK_LAUNCH();
         TRY(pass_x(j, XOP_FWD_COPY, 1, j->S, j->xb, nullptr, nullptr, 0, 0, -1, false));
@@ -638,7 +630,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
         const size_t R = sizeof(float) * (size_t) nv;
         const int fb = (int) std::min<long long>(148 * 16, (nv + 255) / 256);
         if (sl->s.start_condition == DWCU_START_FLAT) {
-            k_fill_scalar<<<fb, 256, 0, st>>>(j->xa, nv, j->sc);
+            k_fill_scalar<<<fb, 256, 0, st>>>(j->xa, nullptr, nv, j->sc);
             CHECK_LAUNCH();
         } else if (sl->s.start_condition == DWCU_START_IDENTITY) {
             CU(cudaMemsetAsync(j->xa, 0, R, st));
@@ -665,6 +657,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
 // iteration k's input transform (iter_input on every part)
 static int slab_input(dwcu_slab *sl, int k)
 {
+    if (k == 0 && sl->s.start_condition == DWCU_START_FLAT) return DWCU_SUCCESS;  // as iter_input
     for (auto &pt : sl->parts) {
         if (!pt.j) continue;
         CU(cudaSetDevice(pt.device));
@@ -680,7 +673,19 @@ static int slab_forward(dwcu_slab *sl, int k, bool ratio)
 {
     const Geometry &g = sl->g;
     const bool shb = (sl->s.method == DWCU_METHOD_SHB);
-    TRY(slab_conv(sl, 0, false, true));
+    if (k == 0 && sl->s.start_condition == DWCU_START_FLAT) {
+        // as iter_forward: every part's image planes
+        for (auto &pt : sl->parts) {
+            if (!pt.j || pt.pl < 1) continue;
+            CU(cudaSetDevice(pt.device));
+            launch_dep(k_flat_rows, dim3((unsigned) ((2 * g.Y + 127) / 128), (unsigned) g.NKB, (unsigned) pt.pl),
+                       dim3(128), 0, pt.stream,
+                       FlatArgs{pt.j->S, pt.j->sc, (int) g.Y, (int) g.NKB, shb ? 1 : 0});
+            CHECK_LAUNCH();
+        }
+    } else {
+        TRY(slab_conv(sl, 0, false, true));
+    }
     const int op = ratio ? (shb ? XOP_RATIO_SHB : XOP_RATIO_RL) : XOP_ERROR_ONLY;
     const long long ytiles = (g.Y + g.xp->R - 1) / g.xp->R;
     for (auto &pt : sl->parts) {
@@ -688,7 +693,7 @@ static int slab_forward(dwcu_slab *sl, int k, bool ratio)
         CU(cudaSetDevice(pt.device));
         const long long tiles = (op == XOP_RATIO_RL) ? pt.j->nxb : pt.pl * ytiles;
         if (tiles > 0) TRY(pass_x(pt.j, op, ratio ? 1 : 0, pt.j->S, nullptr, nullptr, nullptr, 0, 0, tiles));
-        k_slab_err_sum<<<1, kRedThreads, 0, pt.stream>>>(pt.j->partial, (int) tiles, pt.psum + k);
+        k_slab_err_sum<<<1, kErrThreads, 0, pt.stream>>>(pt.j->partial, (int) tiles, pt.psum + k);
         CHECK_LAUNCH();
     }
     if (sl->local >= 0) {

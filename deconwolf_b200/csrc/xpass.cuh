@@ -19,6 +19,7 @@ enum XOp {
     XOP_UPDATE_RL = 7,   // C2R -> x' = clamp(t * (x*W)), store -> [x' -> R2C]
     XOP_WEIGHTS = 8,     // C2R -> W = P1 > 0.01 ? 1/P1 : 0, store
     XOP_STORE = 9,       // C2R -> store real
+    XOP_FWD_PSF = 10,    // the PSF, its peak moved to the origin, scaled -> R2C
 };
 
 struct JobScalars {
@@ -27,8 +28,11 @@ struct JobScalars {
     double sumg;     // sum of the image in double
     float gmin;
     float gmax;      // largest magnitude in the image
+    double psfsum;   // sum of the PSF in double
     int flags;       // bit 0/1: non-finite image/PSF; bits 8+: bounded waits that gave up
 };
+
+struct PsfPeak;
 
 struct XArgs {
     float2 *S;             // spectrum (blocked layout)
@@ -60,6 +64,10 @@ struct XArgs {
     // transform, [wM, wM+hx) and [X-hx, X) take copies of [0, hx) and
     // [wM-hx, wM), the rest of [wM, X) is zero
     int wrapx, wM, hx;
+    // XOP_FWD_PSF: src is the compact PSF, no larger than the volume
+    int pM, pN, pP;
+    const int *peak;       // its first maximum (x, y, z)
+    float scale;
 };
 
 __device__ __forceinline__ float shb_p(float xv, float xpv, double alpha, float bg)
@@ -85,7 +93,7 @@ __device__ __forceinline__ double err_term(float yv, float gv, int metric)
 enum XFam { XFAM_FWD = 0, XFAM_RATIO = 1, XFAM_UPDATE = 2, XFAM_STORE = 3 };
 __host__ __device__ constexpr int x_family(int op)
 {
-    return op <= XOP_FWD_SHBP ? XFAM_FWD
+    return op <= XOP_FWD_SHBP || op == XOP_FWD_PSF ? XFAM_FWD
          : op <= XOP_ERROR_ONLY ? XFAM_RATIO
          : op <= XOP_UPDATE_RL ? XFAM_UPDATE : XFAM_STORE;
 }
@@ -231,6 +239,21 @@ __device__ __forceinline__ void x_row_op(const XArgs &a, int op, int t, long lon
                 const float2 xv = *reinterpret_cast<const float2 *>(sx + c0);
                 const float2 xq = *reinterpret_cast<const float2 *>(sxp + c0);
                 w[r] = make_float2(shb_p(xv.x, xq.x, a.alpha, bg), shb_p(xv.y, xq.y, a.alpha, bg));
+            }
+        }
+        break;
+    case XOP_FWD_PSF:
+        // sx: the PSF row that lands here (null: none); column c holds the
+        // PSF's column (c + peak) mod X
+        if constexpr (FAM == XFAM_FWD) {
+            const int px = a.peak[0];
+#pragma unroll
+            for (int r = 0; r < RL; ++r) {
+                const int c0 = 2 * (t + r * SL);
+                int s0 = c0 + px, s1 = c0 + 1 + px;
+                if (s0 >= 2 * RL * SL) s0 -= 2 * RL * SL;
+                if (s1 >= 2 * RL * SL) s1 -= 2 * RL * SL;
+                w[r] = make_float2(sx && s0 < a.pM ? sx[s0] * a.scale : 0.f, sx && s1 < a.pM ? sx[s1] * a.scale : 0.f);
             }
         }
         break;
@@ -543,6 +566,7 @@ k_xpass(XArgs a)
     const bool row_ok = R == 1 || yy < a.Y;
     const long long plane = (long long) a.nkb * a.Y * KB;  // complex elements per z plane
     const int ks = a.Y * KB;                               // complex elements between kx blocks
+    dep_wait();
 
     if constexpr (FAM == XFAM_RATIO) {
         // (with a periodic x, RL's constant row is not constant over the
@@ -571,6 +595,23 @@ k_xpass(XArgs a)
         }
     }
 
+    const float *psf_row = nullptr;
+    if constexpr (FAM == XFAM_FWD) {
+        if (op == XOP_FWD_PSF) {
+            int sy = yy + a.peak[1], sz = z + a.peak[2];
+            if (sy >= a.Y) sy -= a.Y;
+            if (sz >= a.Z) sz -= a.Z;
+            if (row_ok && sy < a.pN && sz < a.pP) psf_row = a.src + ((long long) sz * a.pN + sy) * a.pM;
+            if (!__syncthreads_or(psf_row != nullptr)) {
+                // no row of this tile holds any of the PSF
+                if (row_ok) {
+                    float2 *Sr = a.S + (long long) z * plane + (long long) yy * KB;
+                    for (int k = t; k <= L; k += TP) Sr[(long long) (k >> 2) * ks + (k & 3)] = make_float2(0.f, 0.f);
+                }
+                return;
+            }
+        }
+    }
     const bool rw = FAM == XFAM_UPDATE && a.Wt != nullptr;
     const bool in_img_row = yy < a.N && z < a.P;
     {
@@ -717,7 +758,8 @@ k_xpass(XArgs a)
             const int j = t + q * TP;
             if (j < SL)
                 x_row_op<FAM, RL, SL>(a, op, j, rbase,
-                                      FAM == XFAM_RATIO ? a.g + ((long long) z * a.N + yy) * a.GP : a.src + rbase,
+                                      FAM == XFAM_RATIO ? a.g + ((long long) z * a.N + yy) * a.GP
+                                      : FAM == XFAM_FWD && op == XOP_FWD_PSF ? psf_row : a.src + rbase,
                                       a.srcp + rbase, rw ? a.Wt + rbase : nullptr, in_img_row, bg, w[q], acc);
         }
     }
@@ -795,6 +837,7 @@ k_xpass(XArgs a)
 #pragma unroll
         for (int q = 0; q < XL::QP; ++q) tx[q] = __ldg(&a.tw[t + q * TP < XL::NP ? t + q * TP : 0]);
         row_sync<TP, R>(row);
+        dep_start_next();
         // last stage: both butterflies of a mirrored pair.  Butterfly M-p's
         // twiddles are W_L^{r(M-p)} = conj(w_r) e^{-2 pi i r/RA} with w_r those
         // of butterfly p; the second factor shifts the outputs by one.
