@@ -31,6 +31,7 @@
 #include "../../include/dwcu.h"
 #include "misc_kernels.cuh"
 #include "launch.cuh"
+#include "hostcopy.h"
 #include "plans_gen.h"
 
 namespace dwcu {
@@ -492,6 +493,59 @@ static void block_put(Block *b)
     for (auto *d : drop) block_free(d);
 }
 
+// for the library's other translation units: a cached block's memory
+void *pool_take(int device, size_t bytes, char **ptr)
+{
+    Block *b = block_get(device, bytes);
+    *ptr = b ? b->ptr : nullptr;
+    return b;
+}
+void pool_give(void *block) { block_put((Block *) block); }
+
+// ------------------------------------------------------------ error slots
+//
+// Page-locked slots that REL / ABS jobs read their errors through: an
+// allocation and its release cost about a millisecond, so released arrays
+// are kept (a few, of at least kSlotFloats floats; dwcu_release_cache frees
+// them).
+constexpr size_t kSlotFloats = 1024, kMaxSlots = 64;
+static std::mutex g_slot_mu;
+static std::vector<std::pair<size_t, float *>> g_slots;
+
+static float *slots_get(size_t n, size_t *have)
+{
+    {
+        std::lock_guard<std::mutex> lk(g_slot_mu);
+        for (size_t i = 0; i < g_slots.size(); ++i)
+            if (g_slots[i].first >= n) {
+                float *p = g_slots[i].second;
+                *have = g_slots[i].first;
+                g_slots.erase(g_slots.begin() + (long) i);
+                return p;
+            }
+    }
+    float *p = nullptr;
+    *have = std::max(n, kSlotFloats);
+    if (cudaHostAlloc(&p, sizeof(float) * *have, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+static void slots_put(float *p, size_t have)
+{
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lk(g_slot_mu);
+        if (g_slots.size() < kMaxSlots) {
+            g_slots.emplace_back(have, p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
 // ------------------------------------------------------------ host iterator
 
 // dw_iterator_t and dw_iterator_{new,next,set_error} (src/dw.h:298-306,
@@ -578,6 +632,7 @@ struct dwcu_job {
     // stopping rules that read the error (REL / ABS): the error values come
     // back into page-locked slots, one per iteration, each marked by an event
     float *h_err = nullptr;
+    size_t h_err_have = 0;
     cudaEvent_t ev_rb[2] = {nullptr, nullptr};
     int spec = -1;                 // iteration whose forward half is queued ahead of its decision
     long long x_pitch = 0;         // pitch of the x pass's real rows (0: the geometry's XP)
@@ -1253,7 +1308,7 @@ static int job_create(long long M, long long N, long long P, long long pM, long 
          cudaEventCreate(&j->ev2) != cudaSuccess))
         rc = fail(DWCU_ERROR_CUDA, "event creation failed");
     if (rc == DWCU_SUCCESS && s->iter_type != DWCU_ITER_FIXED &&
-        (cudaMallocHost(&j->h_err, sizeof(float) * (size_t) trace_cap(*s)) != cudaSuccess ||
+        (!(j->h_err = slots_get((size_t) trace_cap(*s), &j->h_err_have)) ||
          cudaEventCreateWithFlags(&j->ev_rb[0], cudaEventDisableTiming) != cudaSuccess ||
          cudaEventCreateWithFlags(&j->ev_rb[1], cudaEventDisableTiming) != cudaSuccess))
         rc = fail(DWCU_ERROR_CUDA, "error read-back slots could not be set up");
@@ -1275,20 +1330,22 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
     CU(cudaSetDevice(j->s.device));
     cudaStream_t st = j->stream;
     CU(cudaEventRecord(j->ev0, st));
-    const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    // From host memory the image crosses PCIe on the device's copy stream
-    // while the OTF and the weights (which need only the image's size) are
-    // computed; the statistics wait for it (ev2 marks it; the result
-    // records ev2 again).  The PSF goes first: copies in one direction share
-    // one copy engine, and the OTF needs the PSF.
+    // From host memory the PSF goes first; the image crosses PCIe on the
+    // device's copy stream after the OTF and the weights, which need only its
+    // size, have been queued (a copy from pageable memory keeps the host busy
+    // while they run).  The statistics wait for it (ev2 marks it; the result
+    // records ev2 again).
     const long long npsf = g.pM * g.pN * g.pP;
-    CU(cudaMemcpyAsync(j->psf_dev, psf, sizeof(float) * npsf, kind, st));
-    CU(cudaMemsetAsync(j->sc, 0, sizeof(JobScalars), st));
+    const bool from_host = !on_device;
     cudaStream_t cs = on_device ? st : j->ctx->copy;
-    if (cs != st) CU(cudaStreamWaitEvent(cs, j->ev0, 0));
-    CU(cudaMemcpy2DAsync(j->gimg, sizeof(float) * g.GP, im, sizeof(float) * g.M, sizeof(float) * g.M, g.N * g.P,
-                         kind, cs));
-    if (cs != st) CU(cudaEventRecord(j->ev2, cs));
+    if (from_host) {
+        CU(copy_to_device(j->psf_dev, sizeof(float) * npsf, psf, sizeof(float) * npsf, 1, st, j->s.device));
+    } else {
+        CU(cudaMemcpyAsync(j->psf_dev, psf, sizeof(float) * npsf, cudaMemcpyDeviceToDevice, st));
+        CU(cudaMemcpy2DAsync(j->gimg, sizeof(float) * g.GP, im, sizeof(float) * g.M, sizeof(float) * g.M, g.N * g.P,
+                             cudaMemcpyDeviceToDevice, st));
+    }
+    CU(cudaMemsetAsync(j->sc, 0, sizeof(JobScalars), st));
 
     // OTF: PSF with its first maximum at the origin, scaled by 1/(X*Y*Z)
     const long long per = (npsf + j->n_apart - 1) / j->n_apart;
@@ -1344,7 +1401,12 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
     }
 
     // background and start value (the image is on the device from here on)
-    if (cs != st) CU(cudaStreamWaitEvent(st, j->ev2, 0));
+    if (from_host) {
+        CU(cudaStreamWaitEvent(cs, j->ev0, 0));
+        CU(copy_to_device(j->gimg, sizeof(float) * g.GP, im, sizeof(float) * g.M, (size_t) (g.N * g.P), cs, j->s.device));
+        CU(cudaEventRecord(j->ev2, cs));
+        CU(cudaStreamWaitEvent(st, j->ev2, 0));
+    }
     {
         const long long nrows = g.N * g.P;
         const long long rpb = (nrows + j->n_spart - 1) / j->n_spart;
@@ -1630,7 +1692,7 @@ static int job_result(dwcu_job *j, float *out, bool on_device, dwcu_opts *so)
     k_crop<<<fb, 256, 0, st>>>(j->xa, (int) g.XP, (int) g.Y, (int) g.M, (int) g.N, (int) g.P, dout);
     CHECK_LAUNCH();
     CU(cudaEventRecord(j->ev2, st));
-    if (!on_device) CU(cudaMemcpyAsync(out, tmp, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
+    if (!on_device) CU(copy_to_host(out, tmp, sizeof(float) * n, st, j->s.device));
     const int nerr = j->done_iters;
     std::vector<float> errs((size_t) std::max(1, nerr));
     if (nerr > 0) CU(cudaMemcpyAsync(errs.data(), j->err, sizeof(float) * nerr, cudaMemcpyDeviceToHost, st));
@@ -1769,24 +1831,12 @@ static int one_call(const float *im, long long M, long long N, long long P, cons
     TRY(job_create(M, N, P, pM, pN, pP, s, &j));
     if (on_device && stream) j->stream = stream;
     int rc = job_setup(j, im, psf, on_device);
-    // a pageable result buffer is faulted in by a host thread while the
-    // device iterates, so that the result copy does not wait for it
-    std::thread prefault;
-    if (!on_device) {
-        cudaPointerAttributes pa;
-        const bool locked = cudaPointerGetAttributes(&pa, out) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        const size_t n = (size_t) (M * N * P);
-        const uintptr_t o0 = (uintptr_t) out, i0 = (uintptr_t) im, nb = sizeof(float) * n;
-        const bool overlap = o0 < i0 + nb && i0 < o0 + nb;  // an in-place call
-        if (!locked && !overlap && rc == DWCU_SUCCESS)
-            prefault = std::thread([out, n]() {
-                const size_t chunk = (size_t) 1 << 22;
-                for (size_t i = 0; i < n; i += chunk) memset(out + i, 0, sizeof(float) * std::min(chunk, n - i));
-            });
-    }
+    Prefault prefault;
+    const uintptr_t o0 = (uintptr_t) out, i0 = (uintptr_t) im, nb = sizeof(float) * (size_t) (M * N * P);
+    if (!on_device && rc == DWCU_SUCCESS && !(o0 < i0 + nb && i0 < o0 + nb))  // (not the image itself)
+        prefault.start(out, nb);
     if (rc == DWCU_SUCCESS) rc = job_step(j, 1 << 30, nullptr);
-    if (prefault.joinable()) prefault.join();
+    prefault.join();
     if (rc == DWCU_SUCCESS) rc = job_result(j, out, on_device, s);
     if (rc == DWCU_SUCCESS && s->bg_auto) s->bg = j->s.bg;
     dwcu_job_destroy(j);
@@ -2039,6 +2089,16 @@ int dwcu_release_cache(int32_t device)
             kv.second.clear();
         }
     }
+    if (device < 0 || !drop.empty()) {
+        copy_release();
+        std::vector<std::pair<size_t, float *>> slots;
+        {
+            std::lock_guard<std::mutex> lk(g_slot_mu);
+            slots.swap(g_slots);
+        }
+        for (auto &sl : slots) cudaFreeHost(sl.second);
+        cudaGetLastError();
+    }
     int cur = 0;
     const bool had = cudaGetDevice(&cur) == cudaSuccess;
     for (auto *b : drop) {
@@ -2062,7 +2122,7 @@ void dwcu_job_destroy(dwcu_job *j)
     if (j->ev2) cudaEventDestroy(j->ev2);
     for (auto e : j->ev_rb)
         if (e) cudaEventDestroy(e);
-    if (j->h_err) cudaFreeHost(j->h_err);
+    slots_put(j->h_err, j->h_err_have);
     delete j;
 }
 

@@ -153,7 +153,7 @@ X_W = dict(pair=48, mid=11, op=69, sync32=9, sync=30, row=55, latency=8.8)
 def x_R(tp):
     """Rows per tile: one CTA has at least 128 threads up to 32 threads per
     row, two rows above (the error partials are per tile)."""
-    return 2 if tp > 32 else 128 // tp
+    return 1 if tp > 32 else 128 // tp
 
 
 X_TP = [4, 8, 16, 32, 64, 96, 128, 160, 192, 256]

@@ -17,15 +17,22 @@
 #include <cstdio>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <string>
+#include <type_traits>
 #include <thread>
 #include <vector>
 
 #include "../../include/dwcu.h"
+#include "hostcopy.h"
 
 namespace dwcu {
 void record_error(const char *msg);  // engine.cu: the text dwcu_last_error returns
 void record_launch();                // engine.cu: dwcu_launch_count
+// engine.cu: device memory from the cached blocks, given back after the
+// work on it has been waited for
+void *pool_take(int device, size_t bytes, char **ptr);
+void pool_give(void *block);
 }  // namespace dwcu
 
 namespace dwcu_host {
@@ -48,6 +55,29 @@ static int fail(int code, const char *fmt, ...)
             return fail(e_ == cudaErrorMemoryAllocation ? DWCU_ERROR_OUT_OF_MEMORY : DWCU_ERROR_CUDA,  \
                         "%s failed: %s", #call, cudaGetErrorString(e_));                               \
     } while (0)
+
+// device memory for the length of a scope, from the engine's cached blocks
+struct DevBuf {
+    void *block = nullptr;
+    char *ptr = nullptr;
+    bool take(size_t bytes)
+    {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        block = dwcu::pool_take(dev, bytes, &ptr);
+        return block != nullptr;
+    }
+    void give()
+    {
+        if (block) dwcu::pool_give(block);
+        block = nullptr;
+        ptr = nullptr;
+    }
+    DevBuf() = default;
+    DevBuf(const DevBuf &) = delete;
+    DevBuf &operator=(const DevBuf &) = delete;
+    ~DevBuf() { give(); }
+};
 
 // ------------------------------------------------------------ PSF preparation
 
@@ -185,9 +215,21 @@ __global__ void k_psf_plane_sums(const float *__restrict__ p, long long M, long 
 {
     const long long xx = blockIdx.x * (long long) blockDim.x + threadIdx.x;
     if (xx >= M) return;
+    // values loaded a batch ahead, added one by one in the reference's order
+    constexpr int B = 16;
     float sum = 0.f;
-    for (long long yy = 0; yy < N; ++yy)
-        for (long long zz = 0; zz < P; ++zz) sum += p[xx + yy * M + zz * M * N];
+    for (long long yy = 0; yy < N; ++yy) {
+        const float *q = p + xx + yy * M;
+        long long zz = 0;
+        for (; zz + B <= P; zz += B) {
+            float v[B];
+#pragma unroll
+            for (int i = 0; i < B; ++i) v[i] = q[(zz + i) * M * N];
+#pragma unroll
+            for (int i = 0; i < B; ++i) sum += v[i];
+        }
+        for (; zz < P; ++zz) sum += q[zz * M * N];
+    }
     plane[xx] = sum;
 }
 
@@ -219,11 +261,14 @@ static int psf_prepare_device(const float *d_psf, int64_t pM, int64_t pN, int64_
     const size_t o_b1 = o_plane + ((size_t) (4 * pM) + 255) / 256 * 256;
     const size_t o_b2 = o_b1 + ((size_t) (4 * n0) + 255) / 256 * 256;
     const size_t bytes = o_b2 + ((size_t) (4 * n0) + 255) / 256 * 256;
-    HCU(cudaMalloc(&scratch, bytes));
-    struct Free {
-        char *p;
-        ~Free() { cudaFree(p); }
-    } guard{scratch};
+    DevBuf buf;
+    if (!buf.take(bytes)) return fail(DWCU_ERROR_OUT_OF_MEMORY, "PSF scratch");
+    // the block goes back only after the stream's work on it, on every path
+    struct Drain {
+        cudaStream_t st;
+        ~Drain() { cudaStreamSynchronize(st); }
+    } drain{st};
+    scratch = buf.ptr;
     double *part = (double *) (scratch + o_part), *sum1 = (double *) (scratch + o_sum), *sum2 = sum1 + 1;
     long long *first_d = (long long *) (scratch + o_first);
     float *plane = (float *) (scratch + o_plane), *b1 = (float *) (scratch + o_b1), *b2 = (float *) (scratch + o_b2);
@@ -458,11 +503,20 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
         memcpy(ht[(size_t) i].xpos, tiles[(size_t) i].xpos, sizeof ht[0].xpos);
         memcpy(ht[(size_t) i].xsize, tiles[(size_t) i].xsize, sizeof ht[0].xsize);
     }
+    // device memory of the call, given back after its stream has drained
+    DevBuf b_im, b_out, b_tiles, b_psf;
+    std::vector<std::unique_ptr<DevBuf>> b_psfs, b_bufs;
     auto cleanup = [&]() {
-        if (d_im) cudaFree(d_im);
-        if (d_out) cudaFree(d_out);
-        if (d_tiles) cudaFree(d_tiles);
-        if (st) cudaStreamDestroy(st);
+        if (st) {
+            cudaStreamSynchronize(st);
+            cudaStreamDestroy(st);
+        }
+        st = nullptr;
+    };
+    auto take = [](DevBuf &b, size_t bytes, auto **p) {
+        if (!b.take(bytes)) return cudaErrorMemoryAllocation;
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(b.ptr);
+        return cudaSuccess;
     };
 #define TCU(call)                                                                       \
     do {                                                                                \
@@ -473,32 +527,19 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
                         "%s failed: %s", #call, cudaGetErrorString(e_));                \
         }                                                                               \
     } while (0)
-    TCU(cudaMalloc(&d_im, sizeof(float) * nvox));
-    TCU(cudaMalloc(&d_out, sizeof(float) * nvox));
-    TCU(cudaMalloc(&d_tiles, sizeof(DevTile) * (size_t) nt));
-    TCU(cudaMemcpyAsync(d_im, im, sizeof(float) * nvox, cudaMemcpyHostToDevice, st));
+    TCU(take(b_im, sizeof(float) * nvox, &d_im));
+    TCU(take(b_out, sizeof(float) * nvox, &d_out));
+    TCU(take(b_tiles, sizeof(DevTile) * (size_t) nt, &d_tiles));
+    TCU(dwcu::copy_to_device(d_im, sizeof(float) * (size_t) M, im, sizeof(float) * (size_t) M, (size_t) (N * P), st,
+                             s->device));
     TCU(cudaMemcpyAsync(d_tiles, ht.data(), sizeof(DevTile) * (size_t) nt, cudaMemcpyHostToDevice, st));
     TCU(cudaMemsetAsync(d_out, 0, sizeof(float) * nvox, st));
 
-    // Pageable output pages are touched by a host thread while the tiles
-    // iterate, so that the final device-to-host copy does not fault them in
-    // (page-locked memory is resident already).
-    // (not when the result buffer is the image itself)
-    cudaPointerAttributes pa;
-    const bool locked = cudaPointerGetAttributes(&pa, out) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-    cudaGetLastError();
+    // pageable output pages are touched while the tiles iterate (not when the
+    // result buffer is the image itself)
     const uintptr_t o0 = (uintptr_t) out, i0 = (uintptr_t) im, nb = sizeof(float) * nvox;
-    const bool aliased = o0 < i0 + nb && i0 < o0 + nb;
-    std::thread prefault;
-    if (!locked && !aliased)
-        prefault = std::thread([out, nvox]() {
-            const size_t chunk = (size_t) 1 << 22;
-            for (size_t i = 0; i < nvox; i += chunk) memset(out + i, 0, sizeof(float) * std::min(chunk, nvox - i));
-        });
-    struct Joiner {
-        std::thread &t;
-        ~Joiner() { if (t.joinable()) t.join(); }
-    } joiner{prefault};
+    dwcu::Prefault prefault;
+    if (!(o0 < i0 + nb && i0 < o0 + nb)) prefault.start(out, nb);
 
     // per tile: PSF copy normalised and cropped against the tile
     // (dw.c:2112-2130), on the device; tiles of one size share the result
@@ -510,23 +551,9 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
     std::vector<TilePsf> psfs;
     std::vector<int> psf_of((size_t) nt);
     float *d_psf_in = nullptr;
-    auto free_psfs = [&]() {
-        for (auto &tp : psfs)
-            if (tp.dev) cudaFree(tp.dev);
-        if (d_psf_in) cudaFree(d_psf_in);
-        d_psf_in = nullptr;
-    };
-    {
-        cudaError_t e = cudaMalloc(&d_psf_in, sizeof(float) * (size_t) (pM * pN * pP));
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_psf_in, psf, sizeof(float) * (size_t) (pM * pN * pP), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) {
-            free_psfs();
-            cleanup();
-            return fail(e == cudaErrorMemoryAllocation ? DWCU_ERROR_OUT_OF_MEMORY : DWCU_ERROR_CUDA,
-                        "PSF upload failed: %s", cudaGetErrorString(e));
-        }
-    }
+    const size_t psf_bytes = sizeof(float) * (size_t) (pM * pN * pP);
+    TCU(take(b_psf, psf_bytes, &d_psf_in));
+    TCU(dwcu::copy_to_device(d_psf_in, psf_bytes, psf, psf_bytes, 1, st, s->device));
     for (int i = 0; i < nt; ++i) {
         const dwcu_tile &t = tiles[(size_t) i];
         int k = 0;
@@ -536,7 +563,8 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
         if (k == (int) psfs.size()) {
             TilePsf tp;
             memcpy(tp.xs, t.xsize, sizeof tp.xs);
-            int prc = cudaMalloc(&tp.dev, sizeof(float) * (size_t) (pM * pN * pP)) == cudaSuccess
+            b_psfs.emplace_back(new DevBuf());
+            int prc = take(*b_psfs.back(), psf_bytes, &tp.dev) == cudaSuccess
                           ? DWCU_SUCCESS
                           : fail(DWCU_ERROR_OUT_OF_MEMORY, "tile PSF buffer");
             if (prc == DWCU_SUCCESS)
@@ -544,7 +572,6 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
                                          xycropfactor, tp.dev, tp.d, st);
             psfs.push_back(tp);
             if (prc != DWCU_SUCCESS) {
-                free_psfs();
                 cleanup();
                 return prc;
             }
@@ -590,7 +617,8 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
         if (rc) break;
         while (bufs.size() < wave.size()) {
             float *b = nullptr;
-            if (cudaMalloc(&b, sizeof(float) * buf_elems) != cudaSuccess) {
+            b_bufs.emplace_back(new DevBuf());
+            if (take(*b_bufs.back(), sizeof(float) * buf_elems, &b) != cudaSuccess) {
                 rc = fail(DWCU_ERROR_OUT_OF_MEMORY, "tile buffers");
                 break;
             }
@@ -642,14 +670,12 @@ int dwcu_deconvolve_tiled(const float *im, int64_t M, int64_t N, int64_t P, cons
         }
         next = wave.empty() ? nt : wave.back() + 1;
     }
-    if (prefault.joinable()) prefault.join();
+    prefault.join();
     if (rc == DWCU_SUCCESS) {
-        cudaError_t e = cudaMemcpyAsync(out, d_out, sizeof(float) * nvox, cudaMemcpyDeviceToHost, st);
+        cudaError_t e = dwcu::copy_to_host(out, d_out, sizeof(float) * nvox, st, s->device);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "result copy failed: %s", cudaGetErrorString(e));
     }
-    for (auto *b : bufs) cudaFree(b);
-    free_psfs();
     for (auto &T : tj)
         if (T.job) dwcu_job_destroy(T.job);
     cleanup();

@@ -22,12 +22,12 @@ void launch_x_315_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 9, 5>, 
 void launch_x_315_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 7, 5>, 32, 4>(a, st); else launch_x_315_0(a, st); }
 void launch_x_448_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<4, 8, 14>, 32, 4>(a, st); }
 void launch_x_448_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 4, 14>, 32, 4>(a, st); else launch_x_448_0(a, st); }
-void launch_x_640_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 8, 10>, 64, 2>(a, st); }
-void launch_x_640_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<4, 16, 10>, 64, 2>(a, st); else launch_x_640_0(a, st); }
-void launch_x_864_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 9>, 96, 2>(a, st); }
-void launch_x_864_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 16, 9>, 96, 2>(a, st); else launch_x_864_0(a, st); }
-void launch_x_1152_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 12>, 96, 2>(a, st); }
-void launch_x_1152_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 16, 12>, 96, 2>(a, st); else launch_x_1152_0(a, st); }
-void launch_x_1568_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 14, 14>, 128, 2>(a, st); }
-void launch_x_1568_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 16, 14>, 128, 2>(a, st); else launch_x_1568_0(a, st); }
+void launch_x_640_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 8, 10>, 64, 1>(a, st); }
+void launch_x_640_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<4, 16, 10>, 64, 1>(a, st); else launch_x_640_0(a, st); }
+void launch_x_864_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 9>, 96, 1>(a, st); }
+void launch_x_864_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 16, 9>, 96, 1>(a, st); else launch_x_864_0(a, st); }
+void launch_x_1152_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 12>, 96, 1>(a, st); }
+void launch_x_1152_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 16, 12>, 96, 1>(a, st); else launch_x_1152_0(a, st); }
+void launch_x_1568_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 14, 14>, 128, 1>(a, st); }
+void launch_x_1568_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 16, 14>, 128, 1>(a, st); else launch_x_1568_0(a, st); }
 }  // namespace dwcu

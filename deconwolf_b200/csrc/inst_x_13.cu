@@ -22,14 +22,14 @@ void launch_x_280_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<2, 14, 10>
 void launch_x_280_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 4, 10>, 32, 4>(a, st); else launch_x_280_0(a, st); }
 void launch_x_405_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 3, 15>, 32, 4>(a, st); }
 void launch_x_405_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<3, 9, 15>, 32, 4>(a, st); else launch_x_405_0(a, st); }
-void launch_x_576_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<6, 12, 8>, 96, 2>(a, st); }
-void launch_x_576_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 8, 9>, 64, 2>(a, st); else launch_x_576_0(a, st); }
-void launch_x_784_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<4, 14, 14>, 64, 2>(a, st); }
-void launch_x_784_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 8, 14>, 64, 2>(a, st); else launch_x_784_0(a, st); }
-void launch_x_1080_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<6, 15, 12>, 96, 2>(a, st); }
-void launch_x_1080_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 10, 12>, 128, 2>(a, st); else launch_x_1080_0(a, st); }
-void launch_x_1470_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 15, 14>, 128, 2>(a, st); }
-void launch_x_1470_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 14, 15>, 128, 2>(a, st); else launch_x_1470_0(a, st); }
-void launch_x_2016_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 16, 14>, 160, 2>(a, st); }
-void launch_x_2016_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 14, 16>, 160, 2>(a, st); else launch_x_2016_0(a, st); }
+void launch_x_576_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<6, 12, 8>, 96, 1>(a, st); }
+void launch_x_576_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 8, 9>, 64, 1>(a, st); else launch_x_576_0(a, st); }
+void launch_x_784_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<4, 14, 14>, 64, 1>(a, st); }
+void launch_x_784_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 8, 14>, 64, 1>(a, st); else launch_x_784_0(a, st); }
+void launch_x_1080_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<6, 15, 12>, 96, 1>(a, st); }
+void launch_x_1080_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 10, 12>, 128, 1>(a, st); else launch_x_1080_0(a, st); }
+void launch_x_1470_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 15, 14>, 128, 1>(a, st); }
+void launch_x_1470_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 14, 15>, 128, 1>(a, st); else launch_x_1470_0(a, st); }
+void launch_x_2016_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 16, 14>, 160, 1>(a, st); }
+void launch_x_2016_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<9, 14, 16>, 160, 1>(a, st); else launch_x_2016_0(a, st); }
 }  // namespace dwcu

@@ -19,15 +19,15 @@ void launch_x_140_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 2, 10>,
 void launch_x_140_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<2, 7, 10>, 16, 8>(a, st); else launch_x_140_0(a, st); }
 void launch_x_225_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 5, 9>, 32, 4>(a, st); }
 void launch_x_225_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 9, 5>, 32, 4>(a, st); else launch_x_225_0(a, st); }
-void launch_x_343_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 7, 7>, 64, 2>(a, st); }
-void launch_x_490_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 7, 10>, 64, 2>(a, st); }
-void launch_x_490_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 14, 7>, 96, 2>(a, st); else launch_x_490_0(a, st); }
-void launch_x_686_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 14, 7>, 128, 2>(a, st); }
-void launch_x_686_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 7, 14>, 64, 2>(a, st); else launch_x_686_0(a, st); }
-void launch_x_945_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 7, 15>, 96, 2>(a, st); }
-void launch_x_945_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 15, 9>, 128, 2>(a, st); else launch_x_945_0(a, st); }
-void launch_x_1260_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 15, 12>, 128, 2>(a, st); }
-void launch_x_1260_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 15, 14>, 128, 2>(a, st); else launch_x_1260_0(a, st); }
-void launch_x_1680_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 15, 14>, 128, 2>(a, st); }
-void launch_x_1680_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 15>, 128, 2>(a, st); else launch_x_1680_0(a, st); }
+void launch_x_343_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 7, 7>, 64, 1>(a, st); }
+void launch_x_490_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 7, 10>, 64, 1>(a, st); }
+void launch_x_490_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 14, 7>, 96, 1>(a, st); else launch_x_490_0(a, st); }
+void launch_x_686_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 14, 7>, 128, 1>(a, st); }
+void launch_x_686_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 7, 14>, 64, 1>(a, st); else launch_x_686_0(a, st); }
+void launch_x_945_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 7, 15>, 96, 1>(a, st); }
+void launch_x_945_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<7, 15, 9>, 128, 1>(a, st); else launch_x_945_0(a, st); }
+void launch_x_1260_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 15, 12>, 128, 1>(a, st); }
+void launch_x_1260_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<6, 15, 14>, 128, 1>(a, st); else launch_x_1260_0(a, st); }
+void launch_x_1680_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 15, 14>, 128, 1>(a, st); }
+void launch_x_1680_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 15>, 128, 1>(a, st); else launch_x_1680_0(a, st); }
 }  // namespace dwcu

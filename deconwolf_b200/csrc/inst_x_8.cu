@@ -21,13 +21,13 @@ void launch_x_245_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 7, 5>, 
 void launch_x_245_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 7, 7>, 32, 4>(a, st); else launch_x_245_0(a, st); }
 void launch_x_375_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<5, 5, 15>, 32, 4>(a, st); }
 void launch_x_375_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<5, 15, 5>, 32, 4>(a, st); else launch_x_375_0(a, st); }
-void launch_x_512_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 8, 8>, 64, 2>(a, st); }
-void launch_x_512_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<4, 16, 8>, 64, 2>(a, st); else launch_x_512_0(a, st); }
-void launch_x_729_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 9, 9>, 96, 2>(a, st); }
-void launch_x_980_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 14, 10>, 128, 2>(a, st); }
-void launch_x_980_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<10, 14, 7>, 96, 2>(a, st); else launch_x_980_0(a, st); }
-void launch_x_1344_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 14>, 128, 2>(a, st); }
-void launch_x_1344_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 12>, 128, 2>(a, st); else launch_x_1344_0(a, st); }
-void launch_x_1792_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 16, 14>, 160, 2>(a, st); }
-void launch_x_1792_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 16>, 128, 2>(a, st); else launch_x_1792_0(a, st); }
+void launch_x_512_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 8, 8>, 64, 1>(a, st); }
+void launch_x_512_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<4, 16, 8>, 64, 1>(a, st); else launch_x_512_0(a, st); }
+void launch_x_729_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<9, 9, 9>, 96, 1>(a, st); }
+void launch_x_980_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<7, 14, 10>, 128, 1>(a, st); }
+void launch_x_980_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<10, 14, 7>, 96, 1>(a, st); else launch_x_980_0(a, st); }
+void launch_x_1344_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 12, 14>, 128, 1>(a, st); }
+void launch_x_1344_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 12>, 128, 1>(a, st); else launch_x_1344_0(a, st); }
+void launch_x_1792_0(const XArgs &a, cudaStream_t st) { launch_x_t<Rad<8, 16, 14>, 160, 1>(a, st); }
+void launch_x_1792_1(const XArgs &a, cudaStream_t st) { if (x_iteration_op(a.op)) launch_x_iter_t<Rad<8, 14, 16>, 128, 1>(a, st); else launch_x_1792_0(a, st); }
 }  // namespace dwcu

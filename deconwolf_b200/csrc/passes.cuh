@@ -295,7 +295,7 @@ k_lines(LinesArgs a)
     using Cfg = LinesCfg<RD, T>;
     float2 *sotf = sm + Cfg::XCH_F2;  // OTF tile [n][col] (convolve modes)
     const int col0 = tile * T;
-    dep_wait();
+    dep_wait();  // (no dep_start_next: ahead of the stores it cost 3 % at z 120)
     if (mode >= LINES_CONV && (T % 2) == 0) {
         // the tile's OTF columns arrive while the forward transform runs:
         // 16-byte pieces (two columns) of each of the N rows
@@ -324,7 +324,6 @@ k_lines(LinesArgs a)
         line_fft<RD, -1, 1>(v, o, t, a.tw, smem);
     constexpr int SL = N / RD::RL;
     if (mode == LINES_FWD || mode == LINES_INV) {
-        dep_start_next();
         if (t < SL && valid_out) {
 #pragma unroll
             for (int r = 0; r < RD::RL; ++r)
@@ -355,7 +354,6 @@ k_lines(LinesArgs a)
     float2 q[1][RV::RL];
     line_fft<RV, +1, 1>(o, q, t, a.tw, smem);
     constexpr int SQ = N / RV::RL;
-    dep_start_next();
     if (t < SQ && valid) {
 #pragma unroll
         for (int r = 0; r < RV::RL; ++r)
