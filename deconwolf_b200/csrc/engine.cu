@@ -614,6 +614,7 @@ struct dwcu_job {
     // iteration state
     dwcu::Iter it;
     int k_next = -1;               // iteration whose forward half runs next; -1: finished
+    dwcu::ErrSum err_due;          // an error the next convolution pass is to form
     bool flat0 = false;            // iteration 0's estimate is the constant x0 (flat start)
     float x0 = 0;
     bool spectrum_ready = false;   // S holds the transform of iteration k_next's input
@@ -680,8 +681,12 @@ static int launch_lines(dwcu_job *j, const LinesPlan *p, const float2 *tw, long 
         a.packed_y = (int) j->g.Y;
         a.packed_stride = (long long) a.packed_row * a.packed_y;
     }
+    if (mode >= LINES_CONV && !planes) {
+        a.es = j->err_due;
+        j->err_due = ErrSum{};
+    }
     long long nb = (long long) a.ntiles * nouter;
-    if (nb > 0x7fffffffLL) return fail(DWCU_ERROR_UNSUPPORTED, "grid too large");
+    if (nb > 0x7ffffffeLL) return fail(DWCU_ERROR_UNSUPPORTED, "grid too large");
     static const char *names[] = {"lines_fwd", "lines_inv", "lines_conv", "lines_conv_conj"};
     char nm[40];
     snprintf(nm, sizeof nm, "%s_%s", names[mode], axis);
@@ -818,11 +823,17 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
     return DWCU_SUCCESS;
 }
 
-static int err_final(dwcu_job *j, int k, long long tiles)
+// error k from the ratio pass's partials: by a launch of its own, or (defer)
+// left to the next convolution pass, which takes j->err_due along
+static int err_final(dwcu_job *j, int k, long long tiles, bool defer)
 {
     const Geometry &g = j->g;
-    launch_dep(k_err_final, dim3(1), dim3(kErrThreads), 0, j->stream,
-               ErrArgs{j->partial, (int) tiles, (double) (g.M * g.N * g.P), j->err + k});
+    const ErrSum e{j->partial, (int) tiles, (double) (g.M * g.N * g.P), j->err + k};
+    if (defer) {
+        j->err_due = e;
+        return DWCU_SUCCESS;
+    }
+    launch_dep(k_err_final, dim3(1), dim3(kErrLanes), 0, j->stream, e);
     CHECK_LAUNCH();
     return DWCU_SUCCESS;
 }
@@ -849,6 +860,8 @@ static int pass_yconv(dwcu_job *j, int conj)
     a.dir = 0;
     a.otf = j->K;
     a.conj = conj;
+    a.es = j->err_due;
+    j->err_due = ErrSum{};
     ProfScope ps(conj ? "y_conv_conj" : "y_conv", 24.0 * (double) g.NKB * KB * g.Y, j->stream);
     g.ytp->launch(a, j->stream);
     CHECK_LAUNCH();
@@ -893,8 +906,9 @@ static int conv_backward(dwcu_job *j)
 
 // forward half of iteration k: y = K p_k, error_k; when `ratio`, also the
 // ratio's transform into S.  The x pass runs the tiles of planes z < P only
-// when nothing reads the other planes (SHB, or the error alone).
-static int iter_forward(dwcu_job *j, int k, bool ratio)
+// when nothing reads the other planes (SHB, or the error alone).  defer_err:
+// the error is formed beside the back-projection, which the caller runs next.
+static int iter_forward(dwcu_job *j, int k, bool ratio, bool defer_err = false)
 {
     const Geometry &g = j->g;
     const bool shb = (j->s.method == DWCU_METHOD_SHB);
@@ -911,7 +925,7 @@ static int iter_forward(dwcu_job *j, int k, bool ratio)
     // planes z >= P are read later by RL, and by a periodic z (its margins)
     const long long tiles = (op == XOP_RATIO_RL || g.wz) ? j->nxb : g.P * ytiles;
     TRY(pass_x(j, op, ratio ? 1 : 0, j->S, nullptr, nullptr, nullptr, 0, 0, tiles));
-    TRY(err_final(j, k, g.P * ytiles));  // the tiles of planes z >= P add nothing
+    TRY(err_final(j, k, g.P * ytiles, defer_err));  // the tiles of planes z >= P add nothing
     return DWCU_SUCCESS;
 }
 
@@ -1507,8 +1521,9 @@ static int job_step_impl(dwcu_job *j, int nmax, int *remaining)
         const bool last = (k == j->it.niter - 1);
         if (!j->spectrum_ready) TRY(iter_input(j, k));
         // SHB's last update is discarded (method_shb.c:385-395): only its error is needed
-        TRY(iter_forward(j, k, !(last && shb)));
-        if (!(last && shb)) TRY(iter_backward(j, k, !last));
+        const bool back = !(last && shb);
+        TRY(iter_forward(j, k, back, back));
+        if (back) TRY(iter_backward(j, k, !last));
         j->spectrum_ready = !last;
         return DWCU_SUCCESS;
     };

@@ -160,8 +160,23 @@ X_TP = [4, 8, 16, 32, 64, 96, 128, 160, 192, 256]
 X_HELD_MAX = 34
 
 
+def x_serial(n, s, tp):
+    """Instructions that one thread runs for its row, the latency of a pass
+    whose rows all run at once."""
+    a, b, c = s
+    last = c if c > 1 else b
+    ceil = lambda x, y: -(-x // y)  # noqa: E731
+    t = ceil(ceil(n // a, 2), tp) * (4 * DFT_COST[a] + a * X_W["pair"])
+    if c > 1:
+        t += ceil(n // b, tp) * 2 * (DFT_COST[b] + b * X_W["mid"])
+    return t + ceil(n // last, tp) * (2 * DFT_COST[last] + last * X_W["op"])
+
+
 def x_ranked(n):
-    """(split, TP) of half length n, cheapest by x_cost first."""
+    """(split, TP) of half length n, best first: by x_cost times the square
+    root of x_serial.  Measured over 16 half lengths of 25 to 486, against
+    x_cost alone: 22 % less time at 128 Ki spectrum elements (where a pass is
+    one wave of rows), 1 % less at 1 Mi, 1 % more at 16 Mi."""
     out = []
     for s in ranked_splits(n):
         if s[0] == 1:
@@ -169,7 +184,7 @@ def x_ranked(n):
         for tp in X_TP:
             cost, held = x_cost(n, s, tp)
             if held <= X_HELD_MAX:
-                out.append((cost, s, tp))
+                out.append((cost * x_serial(n, s, tp) ** 0.5, s, tp))
     return [(s, tp) for _, s, tp in sorted(out)]
 
 

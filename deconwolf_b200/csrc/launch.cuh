@@ -71,7 +71,11 @@ void launch_lines_t(const LinesArgs &a, int nblocks, cudaStream_t st)
     static KernelOnce ko, kp;
     using C = LinesCfg<RD, T>;
     constexpr int tpl = C::THREADS / T;
-    const size_t smem = a.mode >= LINES_CONV ? C::SMEM_BYTES : C::SMEM_FFT;
+    size_t smem = a.mode >= LINES_CONV ? C::SMEM_BYTES : C::SMEM_FFT;
+    if (a.es.part) {  // one block more, with room for its sums
+        ++nblocks;
+        if (smem < sizeof(double) * kErrLanes) smem = sizeof(double) * kErrLanes;
+    }
     if (a.planes || a.packed) {
         ensure_smem(kp, k_lines<RD, T, true>, C::SMEM_BYTES);
         launch_dep(k_lines<RD, T, true>, dim3(nblocks), dim3(T, tpl), smem, st, a);
@@ -106,7 +110,8 @@ void launch_yconv_t(const YArgs &a, cudaStream_t st)
     static KernelOnce ko;
     using C = YConvCfg<RD>;
     ensure_smem(ko, k_yconv<RD>, C::SMEM_BYTES);
-    launch_dep(k_yconv<RD>, dim3(a.ntiles), dim3(KB, C::TPL), C::SMEM_BYTES, st, a);
+    const size_t room = a.es.part && C::SMEM_BYTES < sizeof(double) * kErrLanes ? sizeof(double) * kErrLanes : C::SMEM_BYTES;
+    launch_dep(k_yconv<RD>, dim3(a.ntiles + (a.es.part ? 1 : 0)), dim3(KB, C::TPL), room, st, a);
 }
 
 }  // namespace dwcu

@@ -365,35 +365,11 @@ __global__ void k_crop(const float *__restrict__ x, int X, int Y, int M, int N, 
 
 // finish one iteration's error: mean over the image of the x-pass partials
 // (get_fIdiv dw.c:1492-1524 / get_fMSE dw.c:1461-1490)
-constexpr int kErrThreads = 1024;
-
-// the sum of nb partials by one block of kErrThreads, in a fixed order
-// (valid on thread 0)
-__device__ __forceinline__ double err_block_sum(const double *part, int nb)
+__global__ void __launch_bounds__(kErrLanes) k_err_final(ErrSum e)
 {
-    __shared__ double s[kErrThreads];
-    double v = 0.0;
-    for (int i = threadIdx.x; i < nb; i += kErrThreads) v += part[i];
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = kErrThreads / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-        __syncthreads();
-    }
-    return s[0];
-}
-
-struct ErrArgs {
-    const double *part;
-    int nb;
-    double count;
-    float *out;
-};
-__global__ void __launch_bounds__(kErrThreads) k_err_final(ErrArgs a)
-{
+    __shared__ double s[kErrLanes];
     dep_wait();
-    const double v = err_block_sum(a.part, a.nb);
-    if (threadIdx.x == 0) *a.out = (float) (v / a.count);
+    err_store(e, s, threadIdx.x, kErrLanes);
 }
 
 }  // namespace dwcu

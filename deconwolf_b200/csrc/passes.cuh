@@ -209,6 +209,57 @@ using RevRad = Rad<(RD::THREE ? RD::RC : RD::RB), (RD::THREE ? RD::RB : RD::RA),
 // two rows y, y+1 of one kx block are 64 contiguous bytes for the x pass.
 constexpr int KB = 4;
 
+// ------------------------------------------------------------ error sums
+//
+// The iteration's error is the sum of the ratio pass's partials.  The
+// back-projection's z pass (or single-plane convolution) that follows has one
+// block more to form it, off the chain of passes, where nothing needs it
+// before that: one launch less per iteration (48 x 40 x 10, SHB 10: 2 us of
+// 22 per iteration).
+constexpr int kErrLanes = 1024;
+
+struct ErrSum {
+    const double *part = nullptr;
+    int nb = 0;
+    double count = 1;
+    float *out = nullptr;
+};
+
+// the sum of nb partials by one block of any size, in the fixed order of
+// kErrLanes strided sums and a tree over them (valid on thread 0); s: kErrLanes doubles
+__device__ __forceinline__ double err_block_sum(const double *part, int nb, double *s, int tid, int threads)
+{
+    // eight lanes of a thread at a time, so that their loads overlap
+    constexpr int G = 8;
+    for (int l0 = tid; l0 < kErrLanes; l0 += G * threads) {
+        double v[G];
+#pragma unroll
+        for (int q = 0; q < G; ++q) v[q] = 0.0;
+        for (int i0 = 0; i0 < nb; i0 += kErrLanes) {
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                const int l = l0 + q * threads;
+                if (l < kErrLanes && i0 + l < nb) v[q] += part[i0 + l];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < G; ++q)
+            if (l0 + q * threads < kErrLanes) s[l0 + q * threads] = v[q];
+    }
+    __syncthreads();
+    for (int o = kErrLanes / 2; o > 0; o >>= 1) {
+        for (int l = tid; l < o; l += threads) s[l] += s[l + o];
+        __syncthreads();
+    }
+    return s[0];
+}
+
+__device__ __forceinline__ void err_store(const ErrSum &e, double *s, int tid, int threads)
+{
+    const double v = err_block_sum(e.part, e.nb, s, tid, threads);
+    if (tid == 0) *e.out = (float) (v / e.count);
+}
+
 // ------------------------------------------------------------ k_lines
 
 enum LinesMode { LINES_FWD = 0, LINES_INV = 1, LINES_CONV = 2, LINES_CONV_CONJ = 3 };
@@ -237,6 +288,7 @@ struct LinesArgs {
     long long packed_stride = 0;
     int packed_row = 0;
     int packed_y = 0;  // rows per plane
+    ErrSum es;         // (part not null) formed by the first block
 };
 
 template <class RD, int T>
@@ -263,8 +315,11 @@ k_lines(LinesArgs a)
     extern __shared__ float2 sm[];
     const int line = threadIdx.x;
     const int t = threadIdx.y;
-    const int tile = blockIdx.x % a.ntiles;
-    const long long outer = blockIdx.x / a.ntiles;
+    // (the error's block comes first, so that it is not the launch's tail)
+    const bool es = !PL && a.es.part;
+    const unsigned bx = es ? blockIdx.x - 1 : blockIdx.x;
+    const int tile = bx % a.ntiles;
+    const long long outer = bx / a.ntiles;
     const int col = tile * T + line;
     const bool valid = col < a.ncols;
     const long long off = outer * a.outer_stride + col;
@@ -296,6 +351,10 @@ k_lines(LinesArgs a)
     float2 *sotf = sm + Cfg::XCH_F2;  // OTF tile [n][col] (convolve modes)
     const int col0 = tile * T;
     dep_wait();  // (no dep_start_next: ahead of the stores it cost 3 % at z 120)
+    if (es && blockIdx.x == 0) {
+        err_store(a.es, reinterpret_cast<double *>(sm), t * T + line, LinesCfg<RD, T>::THREADS);
+        return;
+    }
     if (mode >= LINES_CONV && (T % 2) == 0) {
         // the tile's OTF columns arrive while the forward transform runs:
         // 16-byte pieces (two columns) of each of the N rows
@@ -371,6 +430,7 @@ struct YArgs {
     int dir;            // -1 forward, +1 inverse
     const float2 *otf = nullptr;  // convolution (k_yconv): the OTF, same layout as data
     int conj = 0;       // multiply by its conjugate
+    ErrSum es;          // (k_yconv, part not null) formed by the first block
 };
 
 template <class RD>
@@ -497,8 +557,13 @@ k_yconv(YArgs a)
     uint64_t *bar = reinterpret_cast<uint64_t *>(ysm);
     float2 *A = reinterpret_cast<float2 *>(ysm + 64), *B = A + C::BUF_F2;
     const int l = threadIdx.x, t = threadIdx.y;
-    float2 *tile = a.data + (size_t) blockIdx.x * N * KB;
+    const unsigned bx = a.es.part ? blockIdx.x - 1 : blockIdx.x;  // the error's block comes first
+    float2 *tile = a.data + (size_t) bx * N * KB;
     dep_wait();
+    if (a.es.part && blockIdx.x == 0) {
+        err_store(a.es, reinterpret_cast<double *>(ysm), t * KB + l, C::THREADS);
+        return;
+    }
     if (t == 0 && l == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
@@ -507,7 +572,7 @@ k_yconv(YArgs a)
     }
     float2 h[RD::RL];
     if (t < SL) {
-        const float2 *src = a.otf + (size_t) blockIdx.x * N * KB + l;
+        const float2 *src = a.otf + (size_t) bx * N * KB + l;
 #pragma unroll
         for (int r = 0; r < RD::RL; ++r) h[r] = __ldg(&src[(size_t) (t + r * SL) * KB]);
     }

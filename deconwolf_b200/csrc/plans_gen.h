@@ -1995,68 +1995,68 @@ static const XPlan kXPlans[] = {
     {8, 0, 2, 2, 2, 32, XCfg<Rad<2, 2, 2>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 2, 2>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_8_0},
     {9, 0, 3, 3, 1, 32, XCfg<Rad<3, 3, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<3, 3, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_9_0},
     {10, 0, 2, 5, 1, 32, XCfg<Rad<2, 5, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 5, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_10_0},
-    {12, 0, 4, 3, 1, 32, XCfg<Rad<4, 3, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 3, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_12_0},
+    {12, 0, 2, 2, 3, 32, XCfg<Rad<2, 2, 3>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 2, 3>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_12_0},
     {14, 0, 2, 7, 1, 32, XCfg<Rad<2, 7, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_14_0},
     {15, 0, 3, 5, 1, 32, XCfg<Rad<3, 5, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_15_0},
-    {16, 0, 4, 4, 1, 32, XCfg<Rad<4, 4, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_16_0},
-    {18, 0, 3, 6, 1, 32, XCfg<Rad<3, 6, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<3, 6, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_18_0},
+    {16, 0, 2, 2, 4, 32, XCfg<Rad<2, 2, 4>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 2, 4>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_16_0},
+    {18, 0, 2, 3, 3, 16, XCfg<Rad<2, 3, 3>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 3, 3>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_18_0},
     {20, 0, 4, 5, 1, 32, XCfg<Rad<4, 5, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 5, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_20_0},
     {21, 0, 3, 7, 1, 32, XCfg<Rad<3, 7, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<3, 7, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_21_0},
-    {24, 0, 4, 6, 1, 32, XCfg<Rad<4, 6, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 6, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_24_0},
-    {25, 0, 5, 5, 1, 32, XCfg<Rad<5, 5, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_25_0},
+    {24, 0, 2, 4, 3, 16, XCfg<Rad<2, 4, 3>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 3>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_24_0},
+    {25, 0, 5, 5, 1, 16, XCfg<Rad<5, 5, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_25_0},
     {27, 0, 3, 9, 1, 32, XCfg<Rad<3, 9, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_27_0},
     {28, 0, 4, 7, 1, 32, XCfg<Rad<4, 7, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 7, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_28_0},
-    {30, 0, 3, 10, 1, 32, XCfg<Rad<3, 10, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<3, 10, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_30_0},
-    {32, 0, 4, 8, 1, 32, XCfg<Rad<4, 8, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 8, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_32_0},
-    {35, 0, 7, 5, 1, 32, XCfg<Rad<7, 5, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<7, 5, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_35_0},
-    {36, 0, 2, 2, 9, 32, XCfg<Rad<2, 2, 9>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 2, 9>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_36_0},
-    {40, 0, 2, 2, 10, 32, XCfg<Rad<2, 2, 10>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<2, 2, 10>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_40_0},
-    {42, 0, 7, 6, 1, 32, XCfg<Rad<7, 6, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<7, 6, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_42_0},
-    {45, 0, 3, 5, 3, 16, XCfg<Rad<3, 5, 3>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 3>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_45_0},
-    {48, 0, 4, 12, 1, 32, XCfg<Rad<4, 12, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 12, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_48_0},
-    {49, 0, 7, 7, 1, 32, XCfg<Rad<7, 7, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_49_0},
-    {50, 0, 5, 10, 1, 16, XCfg<Rad<5, 10, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_50_0},
+    {30, 0, 3, 5, 2, 16, XCfg<Rad<3, 5, 2>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 2>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_30_0},
+    {32, 0, 2, 4, 4, 16, XCfg<Rad<2, 4, 4>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 4>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_32_0},
+    {35, 0, 5, 7, 1, 16, XCfg<Rad<5, 7, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<5, 7, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_35_0},
+    {36, 0, 3, 2, 6, 16, XCfg<Rad<3, 2, 6>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<3, 2, 6>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_36_0},
+    {40, 0, 4, 2, 5, 16, XCfg<Rad<4, 2, 5>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<4, 2, 5>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_40_0},
+    {42, 0, 3, 2, 7, 16, XCfg<Rad<3, 2, 7>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<3, 2, 7>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_42_0},
+    {45, 0, 3, 5, 3, 8, XCfg<Rad<3, 5, 3>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 3>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_45_0},
+    {48, 0, 4, 2, 6, 16, XCfg<Rad<4, 2, 6>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<4, 2, 6>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_48_0},
+    {49, 0, 7, 7, 1, 16, XCfg<Rad<7, 7, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_49_0},
+    {50, 0, 2, 5, 5, 8, XCfg<Rad<2, 5, 5>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 5, 5>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_50_0},
     {54, 0, 6, 9, 1, 16, XCfg<Rad<6, 9, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<6, 9, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_54_0},
     {56, 0, 2, 4, 7, 16, XCfg<Rad<2, 4, 7>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 7>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_56_0},
-    {60, 0, 4, 15, 1, 32, XCfg<Rad<4, 15, 1>, 4, 32, XFAM_RATIO>::THREADS, XCfg<Rad<4, 15, 1>, 4, 32, XFAM_RATIO>::SMEM_BYTES, launch_x_60_0},
+    {60, 0, 3, 5, 4, 8, XCfg<Rad<3, 5, 4>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 4>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_60_0},
     {63, 0, 7, 9, 1, 16, XCfg<Rad<7, 9, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_63_0},
-    {64, 0, 2, 4, 8, 16, XCfg<Rad<2, 4, 8>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 8>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_64_0},
-    {70, 0, 7, 10, 1, 16, XCfg<Rad<7, 10, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 10, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_70_0},
-    {72, 0, 2, 4, 9, 16, XCfg<Rad<2, 4, 9>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 9>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_72_0},
+    {64, 0, 4, 4, 4, 8, XCfg<Rad<4, 4, 4>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 4>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_64_0},
+    {70, 0, 2, 7, 5, 8, XCfg<Rad<2, 7, 5>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 5>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_70_0},
+    {72, 0, 3, 4, 6, 8, XCfg<Rad<3, 4, 6>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 4, 6>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_72_0},
     {75, 0, 3, 5, 5, 8, XCfg<Rad<3, 5, 5>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 5>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_75_0},
-    {80, 0, 8, 10, 1, 16, XCfg<Rad<8, 10, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<8, 10, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_80_0},
+    {80, 0, 4, 4, 5, 8, XCfg<Rad<4, 4, 5>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 5>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_80_0},
     {81, 0, 3, 9, 3, 8, XCfg<Rad<3, 9, 3>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 3>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_81_0},
-    {84, 0, 7, 12, 1, 16, XCfg<Rad<7, 12, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 12, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_84_0},
+    {84, 0, 2, 7, 6, 8, XCfg<Rad<2, 7, 6>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 6>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_84_0},
     {90, 0, 3, 5, 6, 8, XCfg<Rad<3, 5, 6>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 6>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_90_0},
-    {96, 0, 8, 12, 1, 16, XCfg<Rad<8, 12, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_96_0},
-    {96, 1, 2, 4, 12, 16, XCfg<Rad<2, 4, 12>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 12>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_96_1},
-    {98, 0, 7, 14, 1, 16, XCfg<Rad<7, 14, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_98_0},
-    {98, 1, 7, 2, 7, 16, XCfg<Rad<7, 2, 7>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 2, 7>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_98_1},
-    {100, 0, 5, 5, 4, 8, XCfg<Rad<5, 5, 4>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 4>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_100_0},
-    {100, 1, 2, 5, 10, 8, XCfg<Rad<2, 5, 10>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 5, 10>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_100_1},
-    {105, 0, 7, 15, 1, 16, XCfg<Rad<7, 15, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_105_0},
-    {105, 1, 3, 5, 7, 16, XCfg<Rad<3, 5, 7>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 7>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_105_1},
+    {96, 0, 4, 4, 6, 8, XCfg<Rad<4, 4, 6>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 6>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_96_0},
+    {96, 1, 2, 8, 6, 8, XCfg<Rad<2, 8, 6>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 8, 6>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_96_1},
+    {98, 0, 2, 7, 7, 8, XCfg<Rad<2, 7, 7>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 7>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_98_0},
+    {98, 1, 7, 2, 7, 8, XCfg<Rad<7, 2, 7>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<7, 2, 7>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_98_1},
+    {100, 0, 4, 5, 5, 4, XCfg<Rad<4, 5, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 5, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_100_0},
+    {100, 1, 5, 5, 4, 4, XCfg<Rad<5, 5, 4>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 4>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_100_1},
+    {105, 0, 5, 3, 7, 8, XCfg<Rad<5, 3, 7>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<5, 3, 7>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_105_0},
+    {105, 1, 3, 5, 7, 8, XCfg<Rad<3, 5, 7>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 7>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_105_1},
     {108, 0, 4, 3, 9, 8, XCfg<Rad<4, 3, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 3, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_108_0},
     {108, 1, 3, 4, 9, 8, XCfg<Rad<3, 4, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 4, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_108_1},
     {112, 0, 4, 4, 7, 8, XCfg<Rad<4, 4, 7>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 7>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_112_0},
     {112, 1, 2, 8, 7, 8, XCfg<Rad<2, 8, 7>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 8, 7>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_112_1},
-    {120, 0, 8, 15, 1, 16, XCfg<Rad<8, 15, 1>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 1>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_120_0},
-    {120, 1, 2, 4, 15, 16, XCfg<Rad<2, 4, 15>, 8, 16, XFAM_RATIO>::THREADS, XCfg<Rad<2, 4, 15>, 8, 16, XFAM_RATIO>::SMEM_BYTES, launch_x_120_1},
-    {125, 0, 5, 5, 5, 8, XCfg<Rad<5, 5, 5>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 5>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_125_0},
-    {126, 0, 2, 7, 9, 8, XCfg<Rad<2, 7, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_126_0},
-    {126, 1, 7, 2, 9, 8, XCfg<Rad<7, 2, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<7, 2, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_126_1},
+    {120, 0, 5, 3, 8, 8, XCfg<Rad<5, 3, 8>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<5, 3, 8>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_120_0},
+    {120, 1, 3, 5, 8, 8, XCfg<Rad<3, 5, 8>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 8>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_120_1},
+    {125, 0, 5, 5, 5, 4, XCfg<Rad<5, 5, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_125_0},
+    {126, 0, 3, 7, 6, 4, XCfg<Rad<3, 7, 6>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 7, 6>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_126_0},
+    {126, 1, 3, 6, 7, 4, XCfg<Rad<3, 6, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 6, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_126_1},
     {128, 0, 4, 4, 8, 8, XCfg<Rad<4, 4, 8>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 8>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_128_0},
     {128, 1, 2, 8, 8, 8, XCfg<Rad<2, 8, 8>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 8, 8>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_128_1},
     {135, 0, 5, 3, 9, 8, XCfg<Rad<5, 3, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<5, 3, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_135_0},
     {135, 1, 3, 5, 9, 8, XCfg<Rad<3, 5, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_135_1},
-    {140, 0, 7, 2, 10, 8, XCfg<Rad<7, 2, 10>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<7, 2, 10>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_140_0},
-    {140, 1, 2, 7, 10, 8, XCfg<Rad<2, 7, 10>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 10>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_140_1},
-    {144, 0, 8, 2, 9, 8, XCfg<Rad<8, 2, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<8, 2, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_144_0},
-    {144, 1, 4, 4, 9, 8, XCfg<Rad<4, 4, 9>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<4, 4, 9>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_144_1},
+    {140, 0, 4, 7, 5, 4, XCfg<Rad<4, 7, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 7, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_140_0},
+    {140, 1, 4, 5, 7, 4, XCfg<Rad<4, 5, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 5, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_140_1},
+    {144, 0, 4, 6, 6, 4, XCfg<Rad<4, 6, 6>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 6, 6>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_144_0},
+    {144, 1, 3, 8, 6, 4, XCfg<Rad<3, 8, 6>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 8, 6>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_144_1},
     {147, 0, 3, 7, 7, 4, XCfg<Rad<3, 7, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 7, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_147_0},
     {147, 1, 7, 7, 3, 4, XCfg<Rad<7, 7, 3>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 3>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_147_1},
-    {150, 0, 5, 3, 10, 8, XCfg<Rad<5, 3, 10>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<5, 3, 10>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_150_0},
-    {150, 1, 3, 5, 10, 8, XCfg<Rad<3, 5, 10>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<3, 5, 10>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_150_1},
+    {150, 0, 3, 10, 5, 4, XCfg<Rad<3, 10, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 10, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_150_0},
+    {150, 1, 5, 6, 5, 4, XCfg<Rad<5, 6, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 6, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_150_1},
     {160, 0, 4, 8, 5, 4, XCfg<Rad<4, 8, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 8, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_160_0},
     {160, 1, 4, 5, 8, 4, XCfg<Rad<4, 5, 8>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 5, 8>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_160_1},
     {162, 0, 3, 9, 6, 4, XCfg<Rad<3, 9, 6>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 6>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_162_0},
@@ -2075,8 +2075,8 @@ static const XPlan kXPlans[] = {
     {196, 1, 2, 14, 7, 4, XCfg<Rad<2, 14, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 14, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_196_1},
     {200, 0, 5, 5, 8, 4, XCfg<Rad<5, 5, 8>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 8>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_200_0},
     {200, 1, 5, 10, 4, 4, XCfg<Rad<5, 10, 4>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 4>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_200_1},
-    {210, 0, 7, 2, 15, 8, XCfg<Rad<7, 2, 15>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<7, 2, 15>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_210_0},
-    {210, 1, 2, 7, 15, 8, XCfg<Rad<2, 7, 15>, 16, 8, XFAM_RATIO>::THREADS, XCfg<Rad<2, 7, 15>, 16, 8, XFAM_RATIO>::SMEM_BYTES, launch_x_210_1},
+    {210, 0, 3, 10, 7, 4, XCfg<Rad<3, 10, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 10, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_210_0},
+    {210, 1, 5, 6, 7, 4, XCfg<Rad<5, 6, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 6, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_210_1},
     {216, 0, 3, 9, 8, 4, XCfg<Rad<3, 9, 8>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 8>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_216_0},
     {216, 1, 4, 6, 9, 4, XCfg<Rad<4, 6, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 6, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_216_1},
     {224, 0, 4, 8, 7, 4, XCfg<Rad<4, 8, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 8, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_224_0},
@@ -2087,10 +2087,10 @@ static const XPlan kXPlans[] = {
     {240, 1, 5, 6, 8, 4, XCfg<Rad<5, 6, 8>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 6, 8>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_240_1},
     {243, 0, 3, 9, 9, 4, XCfg<Rad<3, 9, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_243_0},
     {243, 1, 9, 3, 9, 4, XCfg<Rad<9, 3, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<9, 3, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_243_1},
-    {245, 0, 7, 7, 5, 4, XCfg<Rad<7, 7, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_245_0},
-    {245, 1, 5, 7, 7, 4, XCfg<Rad<5, 7, 7>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 7, 7>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_245_1},
-    {250, 0, 5, 5, 10, 4, XCfg<Rad<5, 5, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_250_0},
-    {250, 1, 5, 10, 5, 4, XCfg<Rad<5, 10, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_250_1},
+    {245, 0, 5, 7, 7, 1, XCfg<Rad<5, 7, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 7, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_245_0},
+    {245, 1, 7, 7, 5, 1, XCfg<Rad<7, 7, 5>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 5>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_245_1},
+    {250, 0, 5, 10, 5, 1, XCfg<Rad<5, 10, 5>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 5>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_250_0},
+    {250, 1, 5, 5, 10, 1, XCfg<Rad<5, 5, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_250_1},
     {252, 0, 7, 9, 4, 4, XCfg<Rad<7, 9, 4>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 4>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_252_0},
     {252, 1, 4, 7, 9, 4, XCfg<Rad<4, 7, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 7, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_252_1},
     {256, 0, 4, 8, 8, 4, XCfg<Rad<4, 8, 8>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 8, 8>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_256_0},
@@ -2099,89 +2099,89 @@ static const XPlan kXPlans[] = {
     {270, 1, 5, 6, 9, 4, XCfg<Rad<5, 6, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 6, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_270_1},
     {280, 0, 2, 14, 10, 4, XCfg<Rad<2, 14, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 14, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_280_0},
     {280, 1, 7, 4, 10, 4, XCfg<Rad<7, 4, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 4, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_280_1},
-    {288, 0, 8, 4, 9, 4, XCfg<Rad<8, 4, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<8, 4, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_288_0},
-    {288, 1, 2, 16, 9, 4, XCfg<Rad<2, 16, 9>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 16, 9>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_288_1},
-    {294, 0, 7, 7, 6, 4, XCfg<Rad<7, 7, 6>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 6>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_294_0},
-    {294, 1, 3, 7, 14, 4, XCfg<Rad<3, 7, 14>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 7, 14>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_294_1},
+    {288, 0, 4, 12, 6, 1, XCfg<Rad<4, 12, 6>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 12, 6>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_288_0},
+    {288, 1, 4, 8, 9, 1, XCfg<Rad<4, 8, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 8, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_288_1},
+    {294, 0, 6, 7, 7, 1, XCfg<Rad<6, 7, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 7, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_294_0},
+    {294, 1, 7, 7, 6, 1, XCfg<Rad<7, 7, 6>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 6>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_294_1},
     {300, 0, 3, 10, 10, 4, XCfg<Rad<3, 10, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 10, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_300_0},
     {300, 1, 5, 6, 10, 4, XCfg<Rad<5, 6, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 6, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_300_1},
-    {315, 0, 7, 9, 5, 4, XCfg<Rad<7, 9, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_315_0},
-    {315, 1, 9, 7, 5, 4, XCfg<Rad<9, 7, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<9, 7, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_315_1},
+    {315, 0, 5, 9, 7, 1, XCfg<Rad<5, 9, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 9, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_315_0},
+    {315, 1, 7, 9, 5, 1, XCfg<Rad<7, 9, 5>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 5>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_315_1},
     {320, 0, 8, 4, 10, 4, XCfg<Rad<8, 4, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<8, 4, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_320_0},
     {320, 1, 2, 16, 10, 4, XCfg<Rad<2, 16, 10>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 16, 10>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_320_1},
     {324, 0, 6, 9, 6, 1, XCfg<Rad<6, 9, 6>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 9, 6>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_324_0},
-    {324, 1, 3, 9, 12, 1, XCfg<Rad<3, 9, 12>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 12>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_324_1},
-    {336, 0, 2, 14, 12, 4, XCfg<Rad<2, 14, 12>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 14, 12>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_336_0},
-    {336, 1, 7, 4, 12, 4, XCfg<Rad<7, 4, 12>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 4, 12>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_336_1},
+    {324, 1, 3, 12, 9, 1, XCfg<Rad<3, 12, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<3, 12, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_324_1},
+    {336, 0, 4, 12, 7, 1, XCfg<Rad<4, 12, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 12, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_336_0},
+    {336, 1, 6, 8, 7, 1, XCfg<Rad<6, 8, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 8, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_336_1},
     {343, 0, 7, 7, 7, 1, XCfg<Rad<7, 7, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_343_0},
     {350, 0, 5, 10, 7, 1, XCfg<Rad<5, 10, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_350_0},
-    {350, 1, 5, 14, 5, 1, XCfg<Rad<5, 14, 5>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 14, 5>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_350_1},
-    {360, 0, 6, 5, 12, 4, XCfg<Rad<6, 5, 12>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<6, 5, 12>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_360_0},
-    {360, 1, 2, 15, 12, 4, XCfg<Rad<2, 15, 12>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 15, 12>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_360_1},
-    {375, 0, 5, 5, 15, 4, XCfg<Rad<5, 5, 15>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 15>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_375_0},
-    {375, 1, 5, 15, 5, 4, XCfg<Rad<5, 15, 5>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<5, 15, 5>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_375_1},
+    {350, 1, 5, 14, 5, 1, XCfg<Rad<5, 14, 5>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 14, 5>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_350_1},
+    {360, 0, 5, 12, 6, 1, XCfg<Rad<5, 12, 6>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 12, 6>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_360_0},
+    {360, 1, 6, 10, 6, 1, XCfg<Rad<6, 10, 6>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 10, 6>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_360_1},
+    {375, 0, 5, 15, 5, 1, XCfg<Rad<5, 15, 5>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 15, 5>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_375_0},
+    {375, 1, 5, 5, 15, 1, XCfg<Rad<5, 5, 15>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 5, 15>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_375_1},
     {378, 0, 6, 9, 7, 1, XCfg<Rad<6, 9, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 9, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_378_0},
     {378, 1, 7, 9, 6, 1, XCfg<Rad<7, 9, 6>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 6>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_378_1},
-    {384, 0, 8, 4, 12, 4, XCfg<Rad<8, 4, 12>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<8, 4, 12>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_384_0},
-    {384, 1, 2, 16, 12, 4, XCfg<Rad<2, 16, 12>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 16, 12>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_384_1},
-    {392, 0, 2, 14, 14, 4, XCfg<Rad<2, 14, 14>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 14, 14>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_392_0},
-    {392, 1, 7, 4, 14, 4, XCfg<Rad<7, 4, 14>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<7, 4, 14>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_392_1},
+    {384, 0, 4, 12, 8, 1, XCfg<Rad<4, 12, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 12, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_384_0},
+    {384, 1, 6, 8, 8, 1, XCfg<Rad<6, 8, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 8, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_384_1},
+    {392, 0, 4, 14, 7, 1, XCfg<Rad<4, 14, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 14, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_392_0},
+    {392, 1, 7, 8, 7, 1, XCfg<Rad<7, 8, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 8, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_392_1},
     {400, 0, 5, 10, 8, 1, XCfg<Rad<5, 10, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_400_0},
-    {400, 1, 8, 10, 5, 1, XCfg<Rad<8, 10, 5>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 10, 5>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_400_1},
-    {405, 0, 9, 3, 15, 4, XCfg<Rad<9, 3, 15>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<9, 3, 15>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_405_0},
-    {405, 1, 3, 9, 15, 4, XCfg<Rad<3, 9, 15>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 15>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_405_1},
-    {420, 0, 2, 15, 14, 4, XCfg<Rad<2, 15, 14>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 15, 14>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_420_0},
-    {420, 1, 2, 14, 15, 4, XCfg<Rad<2, 14, 15>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 14, 15>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_420_1},
-    {432, 0, 9, 3, 16, 4, XCfg<Rad<9, 3, 16>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<9, 3, 16>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_432_0},
-    {432, 1, 3, 9, 16, 4, XCfg<Rad<3, 9, 16>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<3, 9, 16>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_432_1},
+    {400, 1, 4, 10, 10, 1, XCfg<Rad<4, 10, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 10, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_400_1},
+    {405, 0, 5, 9, 9, 1, XCfg<Rad<5, 9, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 9, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_405_0},
+    {405, 1, 3, 15, 9, 1, XCfg<Rad<3, 15, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<3, 15, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_405_1},
+    {420, 0, 4, 15, 7, 1, XCfg<Rad<4, 15, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 15, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_420_0},
+    {420, 1, 5, 12, 7, 1, XCfg<Rad<5, 12, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 12, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_420_1},
+    {432, 0, 6, 9, 8, 1, XCfg<Rad<6, 9, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 9, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_432_0},
+    {432, 1, 4, 12, 9, 1, XCfg<Rad<4, 12, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 12, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_432_1},
     {441, 0, 7, 9, 7, 1, XCfg<Rad<7, 9, 7>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 7>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_441_0},
     {441, 1, 7, 7, 9, 1, XCfg<Rad<7, 7, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_441_1},
-    {448, 0, 4, 8, 14, 4, XCfg<Rad<4, 8, 14>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<4, 8, 14>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_448_0},
-    {448, 1, 8, 4, 14, 4, XCfg<Rad<8, 4, 14>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<8, 4, 14>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_448_1},
-    {450, 0, 2, 15, 15, 4, XCfg<Rad<2, 15, 15>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<2, 15, 15>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_450_0},
-    {450, 1, 10, 3, 15, 4, XCfg<Rad<10, 3, 15>, 32, 4, XFAM_RATIO>::THREADS, XCfg<Rad<10, 3, 15>, 32, 4, XFAM_RATIO>::SMEM_BYTES, launch_x_450_1},
+    {448, 0, 4, 14, 8, 1, XCfg<Rad<4, 14, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 14, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_448_0},
+    {448, 1, 7, 8, 8, 1, XCfg<Rad<7, 8, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 8, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_448_1},
+    {450, 0, 5, 10, 9, 1, XCfg<Rad<5, 10, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_450_0},
+    {450, 1, 6, 15, 5, 1, XCfg<Rad<6, 15, 5>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 5>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_450_1},
     {480, 0, 4, 15, 8, 1, XCfg<Rad<4, 15, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 15, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_480_0},
-    {480, 1, 8, 15, 4, 1, XCfg<Rad<8, 15, 4>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 4>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_480_1},
+    {480, 1, 5, 12, 8, 1, XCfg<Rad<5, 12, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 12, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_480_1},
     {486, 0, 6, 9, 9, 1, XCfg<Rad<6, 9, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 9, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_486_0},
-    {486, 1, 9, 6, 9, 1, XCfg<Rad<9, 6, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 6, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_486_1},
-    {490, 0, 7, 7, 10, 1, XCfg<Rad<7, 7, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_490_0},
-    {490, 1, 5, 14, 7, 1, XCfg<Rad<5, 14, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 14, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_490_1},
+    {486, 1, 9, 9, 6, 1, XCfg<Rad<9, 9, 6>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 6>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_486_1},
+    {490, 0, 5, 14, 7, 1, XCfg<Rad<5, 14, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 14, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_490_0},
+    {490, 1, 7, 10, 7, 1, XCfg<Rad<7, 10, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 10, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_490_1},
     {500, 0, 5, 10, 10, 1, XCfg<Rad<5, 10, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_500_0},
     {500, 1, 10, 5, 10, 1, XCfg<Rad<10, 5, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 5, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_500_1},
     {504, 0, 7, 9, 8, 1, XCfg<Rad<7, 9, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_504_0},
-    {504, 1, 8, 7, 9, 1, XCfg<Rad<8, 7, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 7, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_504_1},
+    {504, 1, 4, 14, 9, 1, XCfg<Rad<4, 14, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 14, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_504_1},
     {512, 0, 8, 8, 8, 1, XCfg<Rad<8, 8, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_512_0},
     {512, 1, 4, 16, 8, 1, XCfg<Rad<4, 16, 8>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 16, 8>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_512_1},
     {525, 0, 5, 15, 7, 1, XCfg<Rad<5, 15, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 15, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_525_0},
-    {525, 1, 7, 15, 5, 1, XCfg<Rad<7, 15, 5>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 5>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_525_1},
+    {525, 1, 7, 15, 5, 1, XCfg<Rad<7, 15, 5>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 5>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_525_1},
     {540, 0, 5, 12, 9, 1, XCfg<Rad<5, 12, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 12, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_540_0},
     {540, 1, 6, 10, 9, 1, XCfg<Rad<6, 10, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 10, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_540_1},
     {560, 0, 4, 14, 10, 1, XCfg<Rad<4, 14, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 14, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_560_0},
     {560, 1, 7, 8, 10, 1, XCfg<Rad<7, 8, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 8, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_560_1},
     {567, 0, 7, 9, 9, 1, XCfg<Rad<7, 9, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_567_0},
-    {567, 1, 9, 7, 9, 1, XCfg<Rad<9, 7, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 7, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_567_1},
+    {567, 1, 9, 7, 9, 1, XCfg<Rad<9, 7, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 7, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_567_1},
     {576, 0, 6, 12, 8, 1, XCfg<Rad<6, 12, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 12, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_576_0},
-    {576, 1, 8, 8, 9, 1, XCfg<Rad<8, 8, 9>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 9>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_576_1},
+    {576, 1, 8, 12, 6, 1, XCfg<Rad<8, 12, 6>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 6>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_576_1},
     {588, 0, 6, 14, 7, 1, XCfg<Rad<6, 14, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 14, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_588_0},
     {588, 1, 7, 12, 7, 1, XCfg<Rad<7, 12, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 12, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_588_1},
     {600, 0, 5, 12, 10, 1, XCfg<Rad<5, 12, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 12, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_600_0},
     {600, 1, 6, 10, 10, 1, XCfg<Rad<6, 10, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 10, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_600_1},
-    {630, 0, 7, 9, 10, 1, XCfg<Rad<7, 9, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_630_0},
-    {630, 1, 6, 15, 7, 1, XCfg<Rad<6, 15, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_630_1},
-    {640, 0, 8, 8, 10, 1, XCfg<Rad<8, 8, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_640_0},
-    {640, 1, 4, 16, 10, 1, XCfg<Rad<4, 16, 10>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 16, 10>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_640_1},
+    {630, 0, 6, 15, 7, 1, XCfg<Rad<6, 15, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_630_0},
+    {630, 1, 7, 9, 10, 1, XCfg<Rad<7, 9, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_630_1},
+    {640, 0, 8, 8, 10, 1, XCfg<Rad<8, 8, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_640_0},
+    {640, 1, 8, 10, 8, 1, XCfg<Rad<8, 10, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 10, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_640_1},
     {648, 0, 6, 12, 9, 1, XCfg<Rad<6, 12, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 12, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_648_0},
     {648, 1, 6, 9, 12, 1, XCfg<Rad<6, 9, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 9, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_648_1},
     {672, 0, 6, 14, 8, 1, XCfg<Rad<6, 14, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 14, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_672_0},
-    {672, 1, 4, 14, 12, 1, XCfg<Rad<4, 14, 12>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 14, 12>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_672_1},
+    {672, 1, 7, 12, 8, 1, XCfg<Rad<7, 12, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 12, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_672_1},
     {675, 0, 5, 15, 9, 1, XCfg<Rad<5, 15, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 15, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_675_0},
     {675, 1, 3, 15, 15, 1, XCfg<Rad<3, 15, 15>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<3, 15, 15>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_675_1},
     {686, 0, 7, 14, 7, 1, XCfg<Rad<7, 14, 7>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 7>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_686_0},
     {686, 1, 7, 7, 14, 1, XCfg<Rad<7, 7, 14>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 14>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_686_1},
     {700, 0, 5, 14, 10, 1, XCfg<Rad<5, 14, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 14, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_700_0},
     {700, 1, 7, 10, 10, 1, XCfg<Rad<7, 10, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 10, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_700_1},
-    {720, 0, 4, 15, 12, 1, XCfg<Rad<4, 15, 12>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 15, 12>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_720_0},
-    {720, 1, 6, 12, 10, 1, XCfg<Rad<6, 12, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 12, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_720_1},
+    {720, 0, 6, 12, 10, 1, XCfg<Rad<6, 12, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 12, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_720_0},
+    {720, 1, 6, 15, 8, 1, XCfg<Rad<6, 15, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_720_1},
     {729, 0, 9, 9, 9, 1, XCfg<Rad<9, 9, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_729_0},
     {735, 0, 7, 15, 7, 1, XCfg<Rad<7, 15, 7>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 7>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_735_0},
     {735, 1, 7, 7, 15, 1, XCfg<Rad<7, 7, 15>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 7, 15>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_735_1},
@@ -2189,75 +2189,75 @@ static const XPlan kXPlans[] = {
     {750, 1, 5, 10, 15, 1, XCfg<Rad<5, 10, 15>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 10, 15>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_750_1},
     {756, 0, 6, 14, 9, 1, XCfg<Rad<6, 14, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 14, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_756_0},
     {756, 1, 7, 12, 9, 1, XCfg<Rad<7, 12, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 12, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_756_1},
-    {768, 0, 8, 8, 12, 1, XCfg<Rad<8, 8, 12>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 12>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_768_0},
-    {768, 1, 4, 16, 12, 1, XCfg<Rad<4, 16, 12>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 16, 12>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_768_1},
-    {784, 0, 4, 14, 14, 1, XCfg<Rad<4, 14, 14>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 14, 14>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_784_0},
-    {784, 1, 7, 8, 14, 1, XCfg<Rad<7, 8, 14>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 8, 14>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_784_1},
+    {768, 0, 8, 12, 8, 1, XCfg<Rad<8, 12, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_768_0},
+    {768, 1, 6, 16, 8, 1, XCfg<Rad<6, 16, 8>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 16, 8>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_768_1},
+    {784, 0, 7, 14, 8, 1, XCfg<Rad<7, 14, 8>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 8>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_784_0},
+    {784, 1, 8, 14, 7, 1, XCfg<Rad<8, 14, 7>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 7>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_784_1},
     {800, 0, 8, 10, 10, 1, XCfg<Rad<8, 10, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 10, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_800_0},
     {800, 1, 5, 16, 10, 1, XCfg<Rad<5, 16, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 16, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_800_1},
     {810, 0, 6, 15, 9, 1, XCfg<Rad<6, 15, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_810_0},
-    {810, 1, 9, 6, 15, 1, XCfg<Rad<9, 6, 15>, 64, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 6, 15>, 64, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_810_1},
+    {810, 1, 9, 10, 9, 1, XCfg<Rad<9, 10, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 10, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_810_1},
     {840, 0, 6, 14, 10, 1, XCfg<Rad<6, 14, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 14, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_840_0},
     {840, 1, 7, 12, 10, 1, XCfg<Rad<7, 12, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 12, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_840_1},
     {864, 0, 8, 12, 9, 1, XCfg<Rad<8, 12, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_864_0},
     {864, 1, 6, 16, 9, 1, XCfg<Rad<6, 16, 9>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 16, 9>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_864_1},
     {882, 0, 7, 14, 9, 1, XCfg<Rad<7, 14, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_882_0},
-    {882, 1, 7, 9, 14, 1, XCfg<Rad<7, 9, 14>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 9, 14>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_882_1},
-    {896, 0, 8, 8, 14, 1, XCfg<Rad<8, 8, 14>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 14>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_896_0},
-    {896, 1, 4, 16, 14, 1, XCfg<Rad<4, 16, 14>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<4, 16, 14>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_896_1},
+    {882, 1, 9, 14, 7, 1, XCfg<Rad<9, 14, 7>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 14, 7>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_882_1},
+    {896, 0, 8, 16, 7, 1, XCfg<Rad<8, 16, 7>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 7>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_896_0},
+    {896, 1, 8, 14, 8, 1, XCfg<Rad<8, 14, 8>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 8>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_896_1},
     {900, 0, 6, 15, 10, 1, XCfg<Rad<6, 15, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_900_0},
     {900, 1, 5, 15, 12, 1, XCfg<Rad<5, 15, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 15, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_900_1},
-    {945, 0, 9, 7, 15, 1, XCfg<Rad<9, 7, 15>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 7, 15>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_945_0},
-    {945, 1, 7, 15, 9, 1, XCfg<Rad<7, 15, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_945_1},
+    {945, 0, 7, 15, 9, 1, XCfg<Rad<7, 15, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_945_0},
+    {945, 1, 9, 15, 7, 1, XCfg<Rad<9, 15, 7>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 7>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_945_1},
     {960, 0, 8, 12, 10, 1, XCfg<Rad<8, 12, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_960_0},
     {960, 1, 6, 16, 10, 1, XCfg<Rad<6, 16, 10>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 16, 10>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_960_1},
-    {972, 0, 9, 9, 12, 1, XCfg<Rad<9, 9, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_972_0},
-    {972, 1, 9, 12, 9, 1, XCfg<Rad<9, 12, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 12, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_972_1},
+    {972, 0, 9, 12, 9, 1, XCfg<Rad<9, 12, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 12, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_972_0},
+    {972, 1, 9, 9, 12, 1, XCfg<Rad<9, 9, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_972_1},
     {980, 0, 7, 14, 10, 1, XCfg<Rad<7, 14, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_980_0},
-    {980, 1, 10, 14, 7, 1, XCfg<Rad<10, 14, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 14, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_980_1},
+    {980, 1, 10, 14, 7, 1, XCfg<Rad<10, 14, 7>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 14, 7>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_980_1},
     {1000, 0, 10, 10, 10, 1, XCfg<Rad<10, 10, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1000_0},
     {1008, 0, 6, 14, 12, 1, XCfg<Rad<6, 14, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 14, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1008_0},
     {1008, 1, 7, 12, 12, 1, XCfg<Rad<7, 12, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 12, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1008_1},
     {1024, 0, 8, 16, 8, 1, XCfg<Rad<8, 16, 8>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 8>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1024_0},
-    {1024, 1, 8, 8, 16, 1, XCfg<Rad<8, 8, 16>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 16>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1024_1},
+    {1024, 1, 8, 8, 16, 1, XCfg<Rad<8, 8, 16>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 8, 16>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1024_1},
     {1050, 0, 7, 15, 10, 1, XCfg<Rad<7, 15, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1050_0},
-    {1050, 1, 10, 15, 7, 1, XCfg<Rad<10, 15, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 15, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1050_1},
+    {1050, 1, 10, 15, 7, 1, XCfg<Rad<10, 15, 7>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 15, 7>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1050_1},
     {1080, 0, 6, 15, 12, 1, XCfg<Rad<6, 15, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1080_0},
-    {1080, 1, 9, 10, 12, 1, XCfg<Rad<9, 10, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 10, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1080_1},
+    {1080, 1, 8, 15, 9, 1, XCfg<Rad<8, 15, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1080_1},
     {1120, 0, 8, 14, 10, 1, XCfg<Rad<8, 14, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1120_0},
     {1120, 1, 7, 16, 10, 1, XCfg<Rad<7, 16, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 16, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1120_1},
     {1125, 0, 5, 15, 15, 1, XCfg<Rad<5, 15, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<5, 15, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1125_0},
-    {1125, 1, 15, 15, 5, 1, XCfg<Rad<15, 15, 5>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<15, 15, 5>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1125_1},
+    {1125, 1, 15, 15, 5, 1, XCfg<Rad<15, 15, 5>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<15, 15, 5>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1125_1},
     {1134, 0, 9, 14, 9, 1, XCfg<Rad<9, 14, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 14, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1134_0},
-    {1134, 1, 9, 9, 14, 1, XCfg<Rad<9, 9, 14>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 14>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1134_1},
+    {1134, 1, 9, 9, 14, 1, XCfg<Rad<9, 9, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1134_1},
     {1152, 0, 8, 12, 12, 1, XCfg<Rad<8, 12, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1152_0},
     {1152, 1, 6, 16, 12, 1, XCfg<Rad<6, 16, 12>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 16, 12>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1152_1},
     {1176, 0, 7, 14, 12, 1, XCfg<Rad<7, 14, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1176_0},
     {1176, 1, 6, 14, 14, 1, XCfg<Rad<6, 14, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 14, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1176_1},
     {1200, 0, 8, 15, 10, 1, XCfg<Rad<8, 15, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1200_0},
-    {1200, 1, 10, 8, 15, 1, XCfg<Rad<10, 8, 15>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 8, 15>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1200_1},
-    {1215, 0, 9, 9, 15, 1, XCfg<Rad<9, 9, 15>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 15>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1215_0},
-    {1215, 1, 9, 15, 9, 1, XCfg<Rad<9, 15, 9>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 9>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1215_1},
+    {1200, 1, 10, 12, 10, 1, XCfg<Rad<10, 12, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 12, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1200_1},
+    {1215, 0, 9, 15, 9, 1, XCfg<Rad<9, 15, 9>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 9>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1215_0},
+    {1215, 1, 9, 9, 15, 1, XCfg<Rad<9, 9, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1215_1},
     {1260, 0, 7, 15, 12, 1, XCfg<Rad<7, 15, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1260_0},
     {1260, 1, 6, 15, 14, 1, XCfg<Rad<6, 15, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1260_1},
     {1280, 0, 8, 16, 10, 1, XCfg<Rad<8, 16, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1280_0},
-    {1280, 1, 10, 8, 16, 1, XCfg<Rad<10, 8, 16>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 8, 16>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1280_1},
+    {1280, 1, 10, 16, 8, 1, XCfg<Rad<10, 16, 8>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 16, 8>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1280_1},
     {1296, 0, 9, 12, 12, 1, XCfg<Rad<9, 12, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 12, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1296_0},
-    {1296, 1, 9, 9, 16, 1, XCfg<Rad<9, 9, 16>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 9, 16>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1296_1},
-    {1344, 0, 8, 12, 14, 1, XCfg<Rad<8, 12, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1344_0},
-    {1344, 1, 8, 14, 12, 1, XCfg<Rad<8, 14, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1344_1},
+    {1296, 1, 9, 16, 9, 1, XCfg<Rad<9, 16, 9>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 16, 9>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1296_1},
+    {1344, 0, 8, 14, 12, 1, XCfg<Rad<8, 14, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1344_0},
+    {1344, 1, 8, 12, 14, 1, XCfg<Rad<8, 12, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1344_1},
     {1350, 0, 6, 15, 15, 1, XCfg<Rad<6, 15, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<6, 15, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1350_0},
-    {1350, 1, 9, 10, 15, 1, XCfg<Rad<9, 10, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 10, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1350_1},
+    {1350, 1, 9, 15, 10, 1, XCfg<Rad<9, 15, 10>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 10>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1350_1},
     {1372, 0, 7, 14, 14, 1, XCfg<Rad<7, 14, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1372_0},
-    {1372, 1, 14, 14, 7, 1, XCfg<Rad<14, 14, 7>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<14, 14, 7>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1372_1},
+    {1372, 1, 14, 14, 7, 1, XCfg<Rad<14, 14, 7>, 256, 1, XFAM_RATIO>::THREADS, XCfg<Rad<14, 14, 7>, 256, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1372_1},
     {1400, 0, 10, 14, 10, 1, XCfg<Rad<10, 14, 10>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 14, 10>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1400_0},
-    {1400, 1, 10, 10, 14, 1, XCfg<Rad<10, 10, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1400_1},
+    {1400, 1, 10, 10, 14, 1, XCfg<Rad<10, 10, 14>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 14>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1400_1},
     {1440, 0, 8, 15, 12, 1, XCfg<Rad<8, 15, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1440_0},
     {1440, 1, 8, 12, 15, 1, XCfg<Rad<8, 12, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 12, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1440_1},
     {1470, 0, 7, 15, 14, 1, XCfg<Rad<7, 15, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1470_0},
     {1470, 1, 7, 14, 15, 1, XCfg<Rad<7, 14, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 14, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1470_1},
     {1500, 0, 10, 15, 10, 1, XCfg<Rad<10, 15, 10>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 15, 10>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1500_0},
-    {1500, 1, 10, 10, 15, 1, XCfg<Rad<10, 10, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1500_1},
+    {1500, 1, 10, 10, 15, 1, XCfg<Rad<10, 10, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1500_1},
     {1512, 0, 9, 14, 12, 1, XCfg<Rad<9, 14, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 14, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1512_0},
     {1512, 1, 9, 12, 14, 1, XCfg<Rad<9, 12, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 12, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1512_1},
     {1536, 0, 8, 16, 12, 1, XCfg<Rad<8, 16, 12>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 12>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1536_0},
@@ -2265,11 +2265,11 @@ static const XPlan kXPlans[] = {
     {1568, 0, 8, 14, 14, 1, XCfg<Rad<8, 14, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1568_0},
     {1568, 1, 7, 16, 14, 1, XCfg<Rad<7, 16, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 16, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1568_1},
     {1575, 0, 7, 15, 15, 1, XCfg<Rad<7, 15, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<7, 15, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1575_0},
-    {1575, 1, 15, 15, 7, 1, XCfg<Rad<15, 15, 7>, 96, 1, XFAM_RATIO>::THREADS, XCfg<Rad<15, 15, 7>, 96, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1575_1},
+    {1575, 1, 15, 15, 7, 1, XCfg<Rad<15, 15, 7>, 256, 1, XFAM_RATIO>::THREADS, XCfg<Rad<15, 15, 7>, 256, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1575_1},
     {1600, 0, 10, 16, 10, 1, XCfg<Rad<10, 16, 10>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 16, 10>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1600_0},
-    {1600, 1, 10, 10, 16, 1, XCfg<Rad<10, 10, 16>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 16>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1600_1},
-    {1620, 0, 9, 12, 15, 1, XCfg<Rad<9, 12, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 12, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1620_0},
-    {1620, 1, 9, 15, 12, 1, XCfg<Rad<9, 15, 12>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 12>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1620_1},
+    {1600, 1, 10, 10, 16, 1, XCfg<Rad<10, 10, 16>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 10, 16>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1600_1},
+    {1620, 0, 9, 15, 12, 1, XCfg<Rad<9, 15, 12>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 12>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1620_0},
+    {1620, 1, 9, 12, 15, 1, XCfg<Rad<9, 12, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 12, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1620_1},
     {1680, 0, 8, 15, 14, 1, XCfg<Rad<8, 15, 14>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 14>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1680_0},
     {1680, 1, 8, 14, 15, 1, XCfg<Rad<8, 14, 15>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 15>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1680_1},
     {1728, 0, 9, 16, 12, 1, XCfg<Rad<9, 16, 12>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 16, 12>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1728_0},
@@ -2279,19 +2279,19 @@ static const XPlan kXPlans[] = {
     {1792, 0, 8, 16, 14, 1, XCfg<Rad<8, 16, 14>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 14>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1792_0},
     {1792, 1, 8, 14, 16, 1, XCfg<Rad<8, 14, 16>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 14, 16>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1792_1},
     {1800, 0, 8, 15, 15, 1, XCfg<Rad<8, 15, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 15, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1800_0},
-    {1800, 1, 10, 12, 15, 1, XCfg<Rad<10, 12, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 12, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1800_1},
+    {1800, 1, 10, 15, 12, 1, XCfg<Rad<10, 15, 12>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 15, 12>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1800_1},
     {1890, 0, 9, 14, 15, 1, XCfg<Rad<9, 14, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 14, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1890_0},
     {1890, 1, 9, 15, 14, 1, XCfg<Rad<9, 15, 14>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 14>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1890_1},
     {1920, 0, 8, 16, 15, 1, XCfg<Rad<8, 16, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1920_0},
     {1920, 1, 10, 16, 12, 1, XCfg<Rad<10, 16, 12>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 16, 12>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1920_1},
     {1960, 0, 10, 14, 14, 1, XCfg<Rad<10, 14, 14>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<10, 14, 14>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1960_0},
-    {1960, 1, 14, 14, 10, 1, XCfg<Rad<14, 14, 10>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<14, 14, 10>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1960_1},
+    {1960, 1, 14, 14, 10, 1, XCfg<Rad<14, 14, 10>, 256, 1, XFAM_RATIO>::THREADS, XCfg<Rad<14, 14, 10>, 256, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_1960_1},
     {2016, 0, 9, 16, 14, 1, XCfg<Rad<9, 16, 14>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 16, 14>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2016_0},
     {2016, 1, 9, 14, 16, 1, XCfg<Rad<9, 14, 16>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 14, 16>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2016_1},
     {2025, 0, 9, 15, 15, 1, XCfg<Rad<9, 15, 15>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<9, 15, 15>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2025_0},
-    {2025, 1, 15, 15, 9, 1, XCfg<Rad<15, 15, 9>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<15, 15, 9>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2025_1},
+    {2025, 1, 15, 15, 9, 1, XCfg<Rad<15, 15, 9>, 256, 1, XFAM_RATIO>::THREADS, XCfg<Rad<15, 15, 9>, 256, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2025_1},
     {2048, 0, 8, 16, 16, 1, XCfg<Rad<8, 16, 16>, 160, 1, XFAM_RATIO>::THREADS, XCfg<Rad<8, 16, 16>, 160, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2048_0},
-    {2048, 1, 16, 8, 16, 1, XCfg<Rad<16, 8, 16>, 128, 1, XFAM_RATIO>::THREADS, XCfg<Rad<16, 8, 16>, 128, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2048_1},
+    {2048, 1, 16, 16, 8, 1, XCfg<Rad<16, 16, 8>, 256, 1, XFAM_RATIO>::THREADS, XCfg<Rad<16, 16, 8>, 256, 1, XFAM_RATIO>::SMEM_BYTES, launch_x_2048_1},
 };
 static const YPlan kYPlans[] = {
     {2, 0, 2, 1, 1, YCfg<Rad<2, 1, 1>>::THREADS, YCfg<Rad<2, 1, 1>>::SMEM_BYTES, launch_y_2_0},

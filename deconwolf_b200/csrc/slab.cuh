@@ -90,9 +90,10 @@ __global__ void k_slab_psf_embed(const float *__restrict__ psf, int pM, int pN, 
 }
 
 // the sum of a part's tile partials, in the fixed order of k_err_final
-__global__ void __launch_bounds__(kErrThreads) k_slab_err_sum(const double *__restrict__ part, int nb, double *out)
+__global__ void __launch_bounds__(kErrLanes) k_slab_err_sum(const double *__restrict__ part, int nb, double *out)
 {
-    const double v = err_block_sum(part, nb);
+    __shared__ double s[kErrLanes];
+    const double v = err_block_sum(part, nb, s, threadIdx.x, kErrLanes);
     if (threadIdx.x == 0) *out = v;
 }
 
@@ -693,7 +694,7 @@ static int slab_forward(dwcu_slab *sl, int k, bool ratio)
         CU(cudaSetDevice(pt.device));
         const long long tiles = (op == XOP_RATIO_RL) ? pt.j->nxb : pt.pl * ytiles;
         if (tiles > 0) TRY(pass_x(pt.j, op, ratio ? 1 : 0, pt.j->S, nullptr, nullptr, nullptr, 0, 0, tiles));
-        k_slab_err_sum<<<1, kErrThreads, 0, pt.stream>>>(pt.j->partial, (int) tiles, pt.psum + k);
+        k_slab_err_sum<<<1, kErrLanes, 0, pt.stream>>>(pt.j->partial, (int) tiles, pt.psum + k);
         CHECK_LAUNCH();
     }
     if (sl->local >= 0) {

@@ -183,11 +183,11 @@ __device__ __forceinline__ void x_row_op(const XArgs &a, int op, int t, long lon
     // only this family's cases are compiled into the kernel
     if (x_family(op) != FAM) return;
     if constexpr (FAM == XFAM_RATIO) {
-        // The usual case of the I-divergence: every y of this thread is
-        // positive and above the guard, and nothing is near the ends of the
-        // float range.  The three ops then share the quotient and differ
-        // outside the image only, and neither the quotient nor the logarithm
-        // needs a branch.  (Everything else, and the squared error: below.)
+        // The usual case: every y of this thread is positive and above the
+        // guard, and nothing is near the ends of the float range.  The three
+        // ops then share the quotient and differ outside the image only, and
+        // neither the quotient nor the logarithm needs a branch.  (Everything
+        // else: below.)
         float lo = 1.f, hi = 1.f;
 #pragma unroll
         for (int r = 0; r < RL; ++r) {
@@ -197,21 +197,33 @@ __device__ __forceinline__ void x_row_op(const XArgs &a, int op, int t, long lon
             lo = fminf(lo, fminf(w[r].x, w[r].y));
             hi = fmaxf(hi, fmaxf(w[r].x, w[r].y));
         }
-        if (a.metric != 0 && lo > 1e-6f && hi <= kRatioBig && a.sc->gmax <= kRatioBig) {
+        if (lo > 1e-6f && hi <= kRatioBig && a.sc->gmax <= kRatioBig) {
             const float outside = op == XOP_RATIO_RL ? 1e-6f : 0.f;
+            // (one loop per metric: a branch inside it cost 8 % of the pass)
+            auto each = [&](auto idiv) {
 #pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const int c0 = 2 * (t + r * SL);
-                const bool img0 = in_img_row && c0 < M, img1 = in_img_row && c0 + 1 < M;
-                float2 gv = img0 ? *reinterpret_cast<const float2 *>(sx + c0) : make_float2(0.f, 0.f);
-                if (!img1) gv.y = 0.f;
-                const float2 v = div_pair(gv, w[r]);
-                const float2 lg = log_pair(v);
-                // g logf(g/y) - (g - y) where g > 0 (dw.c:1514-1517)
-                if (gv.x > 0.f) acc += (double) gv.x * (double) lg.x - ((double) gv.x - (double) w[r].x);
-                if (gv.y > 0.f) acc += (double) gv.y * (double) lg.y - ((double) gv.y - (double) w[r].y);
-                w[r] = make_float2(img0 ? v.x : outside, img1 ? v.y : outside);
-            }
+                for (int r = 0; r < RL; ++r) {
+                    const int c0 = 2 * (t + r * SL);
+                    const bool img0 = in_img_row && c0 < M, img1 = in_img_row && c0 + 1 < M;
+                    float2 gv = img0 ? *reinterpret_cast<const float2 *>(sx + c0) : make_float2(0.f, 0.f);
+                    if (!img1) gv.y = 0.f;
+                    const float2 v = div_pair(gv, w[r]);
+                    if constexpr (decltype(idiv)::value) {
+                        // g logf(g/y) - (g - y) where g > 0 (dw.c:1514-1517)
+                        const float2 lg = log_pair(v);
+                        if (gv.x > 0.f) acc += (double) gv.x * (double) lg.x - ((double) gv.x - (double) w[r].x);
+                        if (gv.y > 0.f) acc += (double) gv.y * (double) lg.y - ((double) gv.y - (double) w[r].y);
+                    } else {
+                        const double d0 = img0 ? (double) w[r].x - (double) gv.x : 0.0;
+                        const double d1 = img1 ? (double) w[r].y - (double) gv.y : 0.0;
+                        acc += d0 * d0;
+                        acc += d1 * d1;
+                    }
+                    w[r] = make_float2(img0 ? v.x : outside, img1 ? v.y : outside);
+                }
+            };
+            if (a.metric != 0) each(std::true_type{});
+            else each(std::false_type{});
             return;
         }
     }
