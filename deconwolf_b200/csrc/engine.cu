@@ -945,6 +945,13 @@ static int iter_backward(dwcu_job *j, int k, bool next)
     return DWCU_SUCCESS;
 }
 
+// whether a job's first forward convolution is that of a constant (k_flat_rows);
+// a PSF larger than the job is not all in its OTF
+static bool flat_first(const Geometry &g, const dwcu_opts &s)
+{
+    return s.start_condition == DWCU_START_FLAT && g.pM <= g.X && g.pN <= g.Y && g.pP <= g.Z;
+}
+
 // transform of iteration k's input (p_k for SHB, x_k for RL) into S
 static int iter_input(dwcu_job *j, int k)
 {
@@ -972,8 +979,7 @@ static int alloc_job(dwcu_job *j)
 {
     const Geometry &g = j->g;
     const int guard_mode = g_guard_mode.load();
-    // the x pass stages R rows per tile; a partial last tile reads (and
-    // never uses) one row past the end, so every staged array gets a spare row
+    // (a spare row after each array, a spare group after each spectrum)
     const size_t R = sizeof(float) * (size_t) (g.real_elems() + g.XP);
     const size_t C = sizeof(float2) * (size_t) (g.spec_elems() + 8 * KB);
     const size_t G = sizeof(float) * (size_t) (g.GP * g.N * g.P + g.GP);
@@ -1344,6 +1350,7 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
     CU(cudaSetDevice(j->s.device));
     cudaStream_t st = j->stream;
     CU(cudaEventRecord(j->ev0, st));
+    j->err_due = ErrSum{};  // of an earlier run that failed half-way
     // From host memory the PSF goes first; the image crosses PCIe on the
     // device's copy stream after the OTF and the weights, which need only its
     // size, have been queued (a copy from pageable memory keeps the host busy
@@ -1475,8 +1482,8 @@ static int job_setup(dwcu_job *j, const float *im, const float *psf, bool on_dev
                                           (int) g.Y);
         CHECK_LAUNCH();
     }
-    j->flat0 = j->s.start_condition == DWCU_START_FLAT;
-    if (j->s.method == DWCU_METHOD_SHB && !j->flat0)
+    j->flat0 = flat_first(g, j->s);
+    if (j->s.method == DWCU_METHOD_SHB && j->s.start_condition != DWCU_START_FLAT)
         CU(cudaMemcpyAsync(j->xb, j->xa, R, cudaMemcpyDeviceToDevice, st));
 
     // input flags (non-finite values) are checked once, here

@@ -105,34 +105,28 @@ __device__ __forceinline__ void butterfly(float2 (&v)[Q][R], const float2 (&w)[R
 // is its base plus a compile-time multiple, so addressing is one add per
 // access.  Contains __syncthreads(): call uniformly from the whole block; the
 // exchange tiles may be reused by the caller only after another barrier.
-// PREF: load each stage's twiddles before the barrier that precedes the
-// stage (hides their latency; costs registers across the barrier).
 // PP (ping-pong): stage 2 writes a second exchange tile, smem2, so that no
 // barrier is needed between its reads and its writes; stage 3 reads smem2.
 // HOIST: the stage twiddles come from tb2 / tb3 (stage_twiddle_base of
 // stages 2 and 3 for this thread, kept by the caller) instead of the table
-// PAD2: the second exchange (stage-2 writes in runs of RA, stage-3
-// unit-stride reads) is padded like the first; without it its reads are
-// conflict-free.  Measured: unpadded is faster for the x pass (one line per
-// thread row), padded for the y pass (four lines interleaved).
-template <class RD, int DIR, int Q, bool PREF, bool PP, class SM, class SM2, bool HOIST = false, bool PAD2 = true>
+template <class RD, int DIR, int Q, bool PP, class SM, class SM2, bool HOIST = false>
 __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o)[Q][RD::RL], int t,
                                               const float2 *__restrict__ tw, SM smem, SM2 smem2,
                                               float2 tb2 = float2{}, float2 tb3 = float2{});
 
-template <class RD, int DIR, int Q, bool PREF = false, bool PAD2 = true, class SM>
+template <class RD, int DIR, int Q, class SM>
 __device__ __forceinline__ void line_fft(float2 (&v)[Q][RD::RA], float2 (&o)[Q][RD::RL], int t,
                                          const float2 *__restrict__ tw, SM smem)
 {
-    line_fft_impl<RD, DIR, Q, PREF, false, SM, SM, false, PAD2>(v, o, t, tw, smem, smem);
+    line_fft_impl<RD, DIR, Q, false, SM, SM>(v, o, t, tw, smem, smem);
 }
 
-template <class RD, int DIR, int Q, bool PREF, bool PP, class SM, class SM2, bool HOIST, bool PAD2>
+template <class RD, int DIR, int Q, bool PP, class SM, class SM2, bool HOIST>
 __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o)[Q][RD::RL], int t,
                                               const float2 *__restrict__ tw, SM smem, SM2 smem2, float2 tb2,
                                               float2 tb3)
 {
-    constexpr int P2 = PAD2 ? RD::PK : 0;  // padding of the second exchange
+    constexpr int P2 = RD::PK;  // padding of the second exchange
     constexpr int N = RD::N, RA = RD::RA, RB = RD::RB, RC = RD::RC;
     constexpr int M2 = N / RB;  // stage-2 butterflies; read stride, a multiple of RA
     // stage 1 writes t*RA + r  ->  padded t*(RA+PK) + r
@@ -146,7 +140,6 @@ __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o
             for (int r = 0; r < RA; ++r) *smem(q, b1 + r) = v[q][r];
     }
     float2 w2[RB];
-    if (PREF && t < M2) stage_twiddles<N, RA, RB>(w2, t, tw);
     __syncthreads();
     if constexpr (RD::THREE) {
         constexpr int M3 = N / RC;
@@ -161,7 +154,7 @@ __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o
         if constexpr (!PP) __syncthreads();
         if (t < M2) {
             if constexpr (HOIST) stage_twiddles_from<RB>(w2, tb2);
-            else if (!PREF) stage_twiddles<N, RA, RB>(w2, t, tw);
+            else stage_twiddles<N, RA, RB>(w2, t, tw);
             butterfly<RA, RB, DIR, Q>(u, w2);
             const int base = (t / RA) * RA * RB + t % RA;  // writes base + r*RA
             const int b3 = base + P2 * (base / RA);
@@ -171,7 +164,6 @@ __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o
                 for (int r = 0; r < RB; ++r) *smem2(q, b3 + r * (RA + P2)) = u[q][r];
         }
         float2 w3[RC];
-        if (PREF && t < M3) stage_twiddles<N, RA * RB, RC>(w3, t, tw);
         __syncthreads();
         if (t < M3) {
             const int b4 = t + P2 * (t / RA);
@@ -180,7 +172,7 @@ __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o
 #pragma unroll
                 for (int r = 0; r < RC; ++r) o[q][r] = *smem2(q, b4 + r * (M3 + P2 * (M3 / RA)));
             if constexpr (HOIST) stage_twiddles_from<RC>(w3, tb3);
-            else if (!PREF) stage_twiddles<N, RA * RB, RC>(w3, t, tw);
+            else stage_twiddles<N, RA * RB, RC>(w3, t, tw);
             butterfly<RA * RB, RC, DIR, Q>(o, w3);
         }
     } else {
@@ -191,7 +183,7 @@ __device__ __forceinline__ void line_fft_impl(float2 (&v)[Q][RD::RA], float2 (&o
 #pragma unroll
                 for (int r = 0; r < RB; ++r) o[q][r] = *smem(q, b2 + r * (M2 + RD::PK * (M2 / RA)));
             if constexpr (HOIST) stage_twiddles_from<RB>(w2, tb2);
-            else if (!PREF) stage_twiddles<N, RA, RB>(w2, t, tw);
+            else stage_twiddles<N, RA, RB>(w2, t, tw);
             butterfly<RA, RB, DIR, Q>(o, w2);
         }
     }
@@ -511,7 +503,7 @@ k_ypass(YArgs a)
             // reads), stage 2 writes the tile buffer back
             float2 *ex = bufs + (size_t) 2 * C::BUF_F2;
             auto smemx = [&](int q, int i) { return ex + (size_t) i * KB + l0 + q; };
-            line_fft_impl<RD, DIR, Q, false, true, decltype(smemx), decltype(smem), true>(v, o, t, a.tw, smemx,
+            line_fft_impl<RD, DIR, Q, true, decltype(smemx), decltype(smem), true>(v, o, t, a.tw, smemx,
                                                                                           smem, tb2, tb3);
         } else {
             __syncthreads();  // natural-order reads done; the buffer becomes the exchange tile
@@ -590,15 +582,15 @@ k_yconv(YArgs a)
     }
     // three stages: B, then A; the inverse's first stage writes B again while
     // the forward's last may still read A.  Two stages: B, then A.
-    line_fft_impl<RD, -1, 1, false, true, decltype(inB), decltype(inA)>(v, o, t, a.tw, inB, inA);
+    line_fft_impl<RD, -1, 1, true, decltype(inB), decltype(inA)>(v, o, t, a.tw, inB, inA);
     if (t < SL) {
 #pragma unroll
         for (int r = 0; r < RD::RL; ++r) o[0][r] = a.conj ? cmulc_paired(o[0][r], h[r]) : cmul_paired(o[0][r], h[r]);
     }
     if constexpr (RD::THREE)
-        line_fft_impl<RV, +1, 1, false, true, decltype(inB), decltype(inA)>(o, q, t, a.tw, inB, inA);
+        line_fft_impl<RV, +1, 1, true, decltype(inB), decltype(inA)>(o, q, t, a.tw, inB, inA);
     else
-        line_fft_impl<RV, +1, 1, false, true, decltype(inA), decltype(inB)>(o, q, t, a.tw, inA, inB);
+        line_fft_impl<RV, +1, 1, true, decltype(inA), decltype(inB)>(o, q, t, a.tw, inA, inB);
     if (t < SQ) {
 #pragma unroll
         for (int r = 0; r < RV::RL; ++r) tile[(size_t) (t + r * SQ) * KB + l] = q[0][r];

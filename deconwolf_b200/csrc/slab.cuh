@@ -658,7 +658,7 @@ static int slab_setup(dwcu_slab *sl, const float *im, const float *psf)
 // iteration k's input transform (iter_input on every part)
 static int slab_input(dwcu_slab *sl, int k)
 {
-    if (k == 0 && sl->s.start_condition == DWCU_START_FLAT) return DWCU_SUCCESS;  // as iter_input
+    if (k == 0 && flat_first(sl->g, sl->s)) return DWCU_SUCCESS;  // as iter_input
     for (auto &pt : sl->parts) {
         if (!pt.j) continue;
         CU(cudaSetDevice(pt.device));
@@ -674,7 +674,7 @@ static int slab_forward(dwcu_slab *sl, int k, bool ratio)
 {
     const Geometry &g = sl->g;
     const bool shb = (sl->s.method == DWCU_METHOD_SHB);
-    if (k == 0 && sl->s.start_condition == DWCU_START_FLAT) {
+    if (k == 0 && flat_first(sl->g, sl->s)) {
         // as iter_forward: every part's image planes
         for (auto &pt : sl->parts) {
             if (!pt.j || pt.pl < 1) continue;

@@ -77,17 +77,6 @@ __device__ __forceinline__ float shb_p(float xv, float xpv, double alpha, float 
     return p < bg ? bg : p;
 }
 
-__device__ __forceinline__ double err_term(float yv, float gv, int metric)
-{
-    double y = yv, g = gv;
-    if (metric == 0) return (y - g) * (y - g);
-    // dw.c:1514-1517: g*logf(g/y) - (g - y) for y > 0 and g > 0.  The
-    // reference divides in double and rounds to float for logf; the float
-    // division gives the same float except in double-rounding ties.
-    if (yv > 0.f && gv > 0.f) return g * (double) logf(gv / yv) - (g - y);
-    return 0.0;
-}
-
 // ops are compiled in four families, one kernel each, so that every kernel's
 // code stays small: forward-only, ratio/error, update, and C2R-store ops
 enum XFam { XFAM_FWD = 0, XFAM_RATIO = 1, XFAM_UPDATE = 2, XFAM_STORE = 3 };
@@ -98,10 +87,10 @@ __host__ __device__ constexpr int x_family(int op)
          : op <= XOP_UPDATE_RL ? XFAM_UPDATE : XFAM_STORE;
 }
 
-__device__ __forceinline__ bool op_c2r(int op) { return op >= XOP_RATIO_SHB; }
-
-// err_term with the quotient g/y already computed (q is only read when
-// y > 0 and g > 0, where it equals g/y)
+// one voxel's error: squared, or g*logf(g/y) - (g - y) for y > 0 and g > 0
+// (dw.c:1514-1517, which divides in double and rounds to float for logf; the
+// float division gives the same float except in double-rounding ties), with
+// the quotient q = g/y already computed (only read when y > 0 and g > 0)
 __device__ __forceinline__ double err_term_q(float yv, float gv, float q, int metric)
 {
     const double y = yv, g = gv;
@@ -114,7 +103,6 @@ __device__ __forceinline__ bool op_reads_x(int op)
     return op == XOP_FWD_COPY || op == XOP_FWD_SHBP || op == XOP_UPDATE_SHB || op == XOP_UPDATE_RL;
 }
 __device__ __forceinline__ bool op_reads_xp(int op) { return op == XOP_FWD_SHBP || op == XOP_UPDATE_SHB; }
-__device__ __forceinline__ bool op_reads_g(int op) { return op >= XOP_RATIO_SHB && op <= XOP_ERROR_ONLY; }
 
 // Quotients g/d of two lanes: a reciprocal refined by one Newton step, the
 // product, and one correction by its exact residual (Markstein, "Computation
@@ -171,8 +159,9 @@ constexpr int XCH = 4;  // elements whose real inputs an update loads together (
 
 // The pointwise op of one row: w[r] holds z[n] = (x[2n], x[2n+1]) for
 // n = t + r*SL -- the C2R output for the C2R ops -- and is replaced by the
-// values handed to the forward transform.  The row's real inputs are staged
-// in shared memory (sx: x or the image row, sxp: x_{k-1}, sw: weights).
+// values handed to the forward transform.  sx, sxp, sw: the row's real inputs
+// in global memory (x or the image row, x_{k-1}, weights), brought into L2 by
+// an earlier block's prefetch.
 // The switch is outside the element loop so each op is one straight loop.
 template <int FAM, int RL, int SL>
 __device__ __forceinline__ void x_row_op(const XArgs &a, int op, int t, long long rbase, const float *sx,
