@@ -5,7 +5,7 @@
 // stage chunks through page-locked buffers, each keeping two chunks in
 // flight, so the copy runs at the link's rate; a result's pages are also
 // touched (and zeroed by the kernel) by several threads while the device
-// iterates.  1024 x 1024 x 60, SHB 10, from and to NumPy arrays: 77 -> 50 ms.
+// iterates.  1024 x 1024 x 60, SHB 10, from and to NumPy arrays: 75 -> 47 ms.
 //
 // The page-locked buffers (kBuffers x kChunk bytes) are made at the first
 // large copy, serve one copy at a time (a second caller meanwhile takes the

@@ -1,15 +1,15 @@
 // noalloc.cu -- dwcu_fft_r2c_noalloc: the 3-D R2C transform of dwcu_fft_r2c
 // without any device-memory allocation.
 //
-// dwcu_fft_r2c takes its work space with cudaMalloc and returns it with
-// cudaFree on every call.  cudaFree synchronises the whole device, so a
-// caller that keeps other work in flight on other streams of the same GPU
-// (a serving loop that interleaves jobs, a pipeline recording into several
-// streams) stalls on every transform, and a caller running under a fixed
-// device-memory budget (a memory pool that owns the rest of the GPU) may not
-// be able to allocate at all.  This variant uses a fixed work space that is
-// part of the library's device image instead: one file-scope array per
-// device, looked up once with cudaGetSymbolAddress.
+// dwcu_fft_r2c takes its work space from the engine's cached blocks and
+// allocates when none fits, and releasing or replacing blocks (cudaFree)
+// synchronises the whole device.  A caller that keeps other work in flight on
+// other streams of the same GPU (a serving loop that interleaves jobs, a
+// pipeline recording into several streams) must not meet that in the middle,
+// and a caller running under a fixed device-memory budget (a memory pool that
+// owns the rest of the GPU) may not be able to allocate at all.  This variant
+// uses a fixed work space that is part of the library's device image: one
+// file-scope array per device, looked up once with cudaGetSymbolAddress.
 //
 // Limits and rules:
 //   * the work space holds kScratchBytes (32 MiB); transforms that need more

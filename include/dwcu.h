@@ -211,8 +211,9 @@ int dwcu_job_result(dwcu_job *job, float *out, int32_t out_on_device, dwcu_opts 
  * memory per device); dwcu_release_cache frees those. */
 void dwcu_job_destroy(dwcu_job *job);
 /* Free the device blocks the library keeps for reuse on `device` (all
- * devices when negative).  No counterpart in the reference, which allocates
- * per call. */
+ * devices when negative), and with them the page-locked copy buffers and
+ * error slots it keeps.  No counterpart in the reference, which allocates per
+ * call. */
 int dwcu_release_cache(int32_t device);
 /* Use a caller stream (cudaStream_t) for this job's work. */
 int dwcu_job_set_stream(dwcu_job *job, void *stream);
@@ -373,10 +374,10 @@ int dwcu_fft_c2r(const float *d_in, int64_t M, int64_t N, int64_t P, float *d_ou
  * reference (deconwolf's fft.c has no allocation-free transform).  Same
  * transform, arguments and result as dwcu_fft_r2c, but the work space is a
  * fixed 32 MiB array in the library's device image (one per device) instead
- * of a cudaMalloc / cudaFree per call: for callers that cannot allocate
- * (a fixed device-memory budget held by their own pool) or cannot afford the
- * device-wide synchronisation of cudaFree while other streams of the GPU are
- * busy.  Transforms whose spectrum, staged input and twiddle tables need more
+ * of a cached block that is allocated when none fits: for callers that cannot
+ * allocate (a fixed device-memory budget held by their own pool) or cannot
+ * afford the device-wide synchronisation of an allocation's release while
+ * other streams of the GPU are busy.  Transforms whose spectrum, staged input and twiddle tables need more
  * than the work space are rejected with DWCU_ERROR_INVALID_VALUE.  The first
  * call on a device does one-time setup (symbol lookup, kernel attributes),
  * so make that first call before any stream capture.  Calls on one device
