@@ -513,24 +513,59 @@ __device__ __forceinline__ void x_butterfly(float2 *v, const float2 (&w)[R])
     Dft<R, DIR>::run(v);
 }
 
-// The table values a stage's twiddles are powers of (radix RS after NS), for
-// each of this thread's butterflies.  Loaded before the barrier in front of
-// the stage: with most of shared memory in use the tables miss the L1 cache,
-// and behind the barrier every warp of the row would wait for them.
+// A stage's twiddles are the powers w^r, r < RS, of one root: every D-th is
+// loaded from the table, the others are a loaded one times one of the first.
+// Powers of a single value carry its rounding error r times, which is what
+// bounds a transform's accuracy here (the wide radices are in stages that
+// have twiddles): the table values halve or third the chain.  Short rows have
+// few stages to average over and take more of them; their pass is latency
+// bound, where the loads cost nothing.  C2R error in units of 2^-24, half
+// lengths 375 / 420 / 1350: 3.9 / 4.4 / 5.5 with one value, 2.2 / 2.2 / 2.6
+// with these (largest over the 176 lengths and both directions, relative to
+// the square root of the transform's factors of two: 1.62 -> 0.86); x 2240
+// update 4.37 -> 4.45 ms, x 700 0.279 -> 0.290 (RL), whole deconvolutions
+// 0 to 1 % more.
+template <int L, int RS>
+struct XTw {
+    static constexpr int D = L < 128 ? (RS <= 7 ? 2 : 4) : RS <= 4 ? RS : RS <= 10 ? (RS + 1) / 2 : (RS + 2) / 3;
+    static constexpr int NB = 1 + (RS - 1) / D;  // table values: w, w^D, w^2D, ...
+};
+
+// The table values of a stage (radix RS after NS), for each of this thread's
+// butterflies.  Loaded before the barrier in front of the stage: with most of
+// shared memory in use the tables miss the L1 cache, and behind the barrier
+// every warp of the row would wait for them.
 template <int L, int NS, int RS, int TP, int Q>
-__device__ __forceinline__ void x_bases(float2 (&b)[Q], int t, const float2 *__restrict__ tw)
+__device__ __forceinline__ void x_bases(float2 (&b)[Q][XTw<L, RS>::NB], int t, const float2 *__restrict__ tw)
 {
+    constexpr int step = L / (NS * RS);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int j = t + q * TP;
-        b[q] = stage_twiddle_base<L, NS, RS>(j < L / RS ? j : 0, tw);
+        const int u = (j < L / RS ? j % NS : 0) * step;
+        b[q][0] = __ldg(&tw[u]);
+#pragma unroll
+        for (int i = 1; i < XTw<L, RS>::NB; ++i) b[q][i] = __ldg(&tw[u * (i * XTw<L, RS>::D)]);
     }
+}
+
+// the twiddles from those values
+template <int L, int RS>
+__device__ __forceinline__ void x_twiddles(float2 (&w)[RS], const float2 (&b)[XTw<L, RS>::NB])
+{
+    constexpr int D = XTw<L, RS>::D;
+    if constexpr (RS > 1) w[1] = b[0];
+#pragma unroll
+    for (int r = 2; r < RS; ++r)
+        w[r] = r % D == 0 ? b[r / D]
+             : r > D      ? cmul(w[r / D * D], w[r % D])
+             : r % 2 == 0 ? cmul(w[r / 2], w[r / 2]) : cmul(w[r - 1], w[1]);
 }
 
 // middle stage (radix B after a first radix R1): first exchange in, second
 // out; tb: x_bases of the stage
 template <int L, int R1, int B, int DIR, int TP, int Q>
-__device__ __forceinline__ void x_mid(const float2 *in, float2 *out, int t, const float2 (&tb)[Q], int gap)
+__device__ __forceinline__ void x_mid(const float2 *in, float2 *out, int t, const float2 (&tb)[Q][XTw<L, B>::NB], int gap)
 {
     constexpr int M2 = L / B, PK = R1 % 2 == 0 ? 1 : 0;
 #pragma unroll
@@ -541,7 +576,7 @@ __device__ __forceinline__ void x_mid(const float2 *in, float2 *out, int t, cons
             const int b = j + PK * (j / R1);
 #pragma unroll
             for (int r = 0; r < B; ++r) u[r] = in[b + r * (M2 + PK * (M2 / R1))];
-            stage_twiddles_from<B>(w, tb[q]);
+            x_twiddles<L, B>(w, tb[q]);
             x_butterfly<B, DIR>(u, w);
             float2 *o = out + (j / R1) * (R1 * B + gap) + j % R1;
 #pragma unroll
@@ -722,9 +757,9 @@ k_xpass(XArgs a)
             }
         }
         const float2 *in = T0;
-        float2 tl[QL];
+        float2 tl[QL][XTw<L, RL>::NB];
         if constexpr (RD::THREE) {
-            float2 tm[XL::Q2];
+            float2 tm[XL::Q2][XTw<L, RB>::NB];
             x_bases<L, RA, RB, TP>(tm, t, a.twL);
             row_sync<TP, R>(row);
             x_mid<L, RA, RB, +1, TP>(T0, T1, t, tm, XL::gap(RA, RB));
@@ -737,7 +772,7 @@ k_xpass(XArgs a)
             const int j = t + q * TP;
             if (j < SL) {
                 float2 tw[RL];
-                stage_twiddles_from<RL>(tw, tl[q]);
+                x_twiddles<L, RL>(tw, tl[q]);
                 if constexpr (RD::THREE) {
 #pragma unroll
                     for (int r = 0; r < RL; ++r) w[q][r] = in[j + r * (SL + XL::gap(RA, RB))];
@@ -826,9 +861,9 @@ k_xpass(XArgs a)
             }
         }
         const float2 *in = F0;
-        float2 tl[XL::QP], tx[XL::QP];
+        float2 tl[XL::QP][XTw<L, RA>::NB], tx[XL::QP];
         if constexpr (RD::THREE) {
-            float2 tm[XL::Q2];
+            float2 tm[XL::Q2][XTw<L, RB>::NB];
             x_bases<L, RL, RB, TP>(tm, t, a.twL);
             row_sync<TP, R>(row);
             x_mid<L, RL, RB, -1, TP>(F0, F1, t, tm, XL::gap(RL, RB));
@@ -866,7 +901,7 @@ k_xpass(XArgs a)
                     v1[r] = in[at(p, r)];
                     v2[r] = in[at(j2, r)];
                 }
-                stage_twiddles_from<RA>(tw, tl[q]);
+                x_twiddles<L, RA>(tw, tl[q]);
                 x_butterfly<RA, -1>(v1, tw);
                 if (p == 0) {
                     static_for<RA>([&](auto rc) {
