@@ -155,6 +155,14 @@ __device__ __forceinline__ float2 log_pair(float2 q)
 }
 
 constexpr float kRatioBig = 1152921504606846976.f;  // 2^60: the range div_pair is exact in
+
+// the smaller of two values, NaN if either is
+__device__ __forceinline__ float min_nan(float a, float b)
+{
+    float m;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
 constexpr int XCH = 4;  // elements whose real inputs an update loads together (2 and 8: 2-10 % slower)
 
 // The pointwise op of one row: w[r] holds z[n] = (x[2n], x[2n+1]) for
@@ -176,14 +184,14 @@ __device__ __forceinline__ void x_row_op(const XArgs &a, int op, int t, long lon
         // guard, and nothing is near the ends of the float range.  The three
         // ops then share the quotient and differ outside the image only, and
         // neither the quotient nor the logarithm needs a branch.  (Everything
-        // else: below.)
+        // else, NaN among it: below.)
         float lo = 1.f, hi = 1.f;
 #pragma unroll
         for (int r = 0; r < RL; ++r) {
             const int c0 = 2 * (t + r * SL);
             if (!(in_img_row && c0 < M)) w[r].x = 1.f;
             if (!(in_img_row && c0 + 1 < M)) w[r].y = 1.f;
-            lo = fminf(lo, fminf(w[r].x, w[r].y));
+            lo = min_nan(lo, min_nan(w[r].x, w[r].y));
             hi = fmaxf(hi, fmaxf(w[r].x, w[r].y));
         }
         if (lo > 1e-6f && hi <= kRatioBig && a.sc->gmax <= kRatioBig) {
