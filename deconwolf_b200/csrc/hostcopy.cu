@@ -8,8 +8,9 @@
 // iterates.  1024 x 1024 x 60, SHB 10, from and to NumPy arrays: 75 -> 47 ms.
 //
 // The page-locked buffers (kBuffers x kChunk bytes) are made at the first
-// large copy, serve one copy at a time (a second caller meanwhile takes the
-// driver's path rather than wait) and are given back by dwcu_release_cache.
+// large copy, serve one copy at a time for as long as its bytes move (a second
+// caller meanwhile takes the driver's path rather than wait) and are given
+// back by dwcu_release_cache.
 // Page-locked, registered and managed memory, and copies below kMinBytes,
 // take the driver's path, which is at its best there.
 #include <cuda_runtime.h>
@@ -135,6 +136,10 @@ cudaError_t staged(bool to_device, char *host, char *dev, size_t dpitch, size_t 
 {
     *done = false;
     if (row_bytes * rows < kMinBytes || row_bytes > kChunk || !pageable(host)) return cudaSuccess;
+    // what is queued on the stream (a result's whole run of iterations) is
+    // waited for here, by one thread: not with the buffers held, nor by every
+    // worker
+    if (const cudaError_t e = cudaStreamSynchronize(st)) return e;
     std::unique_lock<std::mutex> lk(g_ring_mu, std::try_to_lock);
     if (!lk.owns_lock()) return cudaSuccess;
     char *ring = ring_locked();
