@@ -380,6 +380,7 @@ struct Block {
     char *ptr = nullptr;
     size_t bytes = 0;
     int device = 0;
+    bool work = false;  // last the work space of a call, not a job's memory
     struct Graph {
         cudaGraphExec_t exec = nullptr;
         long long kernels = 0;
@@ -393,6 +394,13 @@ static std::map<int, std::vector<Block *>> g_blk_free;
 // released blocks kept per device: at most this many, and at most half of
 // the device's memory together
 constexpr size_t kMaxCachedBlocks = 64;
+// A call's work space (a transform's spectrum, the tiled call's image, result
+// and tile buffers) is kept too, but no more of it than this share of the
+// device together: a program that transforms volumes of many sizes beside
+// another allocator keeps the rest of the device for that.  An allocation and
+// its release take a millisecond or two whatever their size, which is most of
+// a call that needs megabytes and little of one that needs more than this.
+constexpr double kMaxWorkShare = 1.0 / 32;
 
 static size_t device_total_bytes(int device)
 {
@@ -473,22 +481,37 @@ static Block *block_get(int device, size_t bytes)
     return b;
 }
 
-static void block_put(Block *b)
+static void block_put(Block *b, bool work = false)
 {
     if (!b) return;
+    const double total = (double) device_total_bytes(b->device), share = kMaxWorkShare * total;
+    b->work = work;
+    if (work && (double) b->bytes > share) {
+        block_free(b);
+        return;
+    }
     std::vector<Block *> drop;
     {
         std::lock_guard<std::mutex> lk(g_blk_mu);
         auto &v = g_blk_free[b->device];
         v.push_back(b);
-        const double cap = 0.5 * (double) device_total_bytes(b->device);
-        double held = 0;
-        for (auto *c : v) held += (double) c->bytes;
-        while (!v.empty() && (v.size() > kMaxCachedBlocks || held > cap)) {
-            held -= (double) v.front()->bytes;
-            drop.push_back(v.front());
-            v.erase(v.begin());
+        double held = 0, works = 0;
+        for (auto *c : v) {
+            held += (double) c->bytes;
+            if (c->work) works += (double) c->bytes;
         }
+        // the oldest go first: work space beyond its share, then any block
+        auto drop_at = [&](size_t i) {
+            held -= (double) v[i]->bytes;
+            if (v[i]->work) works -= (double) v[i]->bytes;
+            drop.push_back(v[i]);
+            v.erase(v.begin() + (long) i);
+        };
+        for (size_t i = 0; i < v.size() && works > share;) {
+            if (v[i]->work) drop_at(i);
+            else ++i;
+        }
+        while (!v.empty() && (v.size() > kMaxCachedBlocks || held > 0.5 * total)) drop_at(0);
     }
     for (auto *d : drop) block_free(d);
 }
@@ -500,7 +523,7 @@ void *pool_take(int device, size_t bytes, char **ptr)
     *ptr = b ? b->ptr : nullptr;
     return b;
 }
-void pool_give(void *block) { block_put((Block *) block); }
+void pool_give(void *block) { block_put((Block *) block, true); }
 
 // ------------------------------------------------------------ error slots
 //
@@ -1969,7 +1992,7 @@ static int fft3d(const float *d_in, long long M, long long N, long long P, float
     if (cudaMemsetAsync(j->sc, 0, sizeof(JobScalars), j->stream) != cudaSuccess) rc = fail(DWCU_ERROR_CUDA, "memset");
     if (rc == DWCU_SUCCESS) rc = forward ? fft3d_forward(j, d_in, d_out, real) : fft3d_inverse(j, d_in, d_out, real);
     rc = fft3d_finish(j, rc);
-    block_put(blk);
+    block_put(blk, true);
     j->stream = nullptr;
     return rc;
 }

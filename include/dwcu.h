@@ -208,7 +208,10 @@ int dwcu_job_done(const dwcu_job *job);
 int dwcu_job_result(dwcu_job *job, float *out, int32_t out_on_device, dwcu_opts *s_out);
 /* Release the job.  Its device block is kept by the library for the next
  * job of a similar size (at most 64 blocks and half of the device's
- * memory per device); dwcu_release_cache frees those. */
+ * memory per device); dwcu_release_cache frees those.  The work space of
+ * other calls (the transforms below, dwcu_deconvolve_tiled's image, result,
+ * PSF and tile buffers, dwcu_psf_prepare_device's scratch) is kept among
+ * them, at most a thirty-second of the device's memory together. */
 void dwcu_job_destroy(dwcu_job *job);
 /* Free the device blocks the library keeps for reuse on `device` (all
  * devices when negative), and with them the page-locked copy buffers and
@@ -362,7 +365,9 @@ void dwcu_server_destroy(dwcu_server *server);
 /* 3-D real-to-complex transform of d_in (M x N x P floats, device) into
  * d_out ((M/2+1) x N x P interleaved complex, device), unnormalised, the
  * layout of fftwf_plan_dft_r2c_3d(P, N, M, ...).  Replaces fft() (src/fft.c:
- * 401-415).  M must be even with M/2, N and P supported lengths. */
+ * 401-415).  M must be even with M/2, N and P supported lengths.  The work
+ * space (about the size of d_out) stays in the library's cache after the call
+ * (see dwcu_job_destroy). */
 int dwcu_fft_r2c(const float *d_in, int64_t M, int64_t N, int64_t P, float *d_out, int32_t device,
                  void *stream);
 /* Complex-to-real inverse of the above, unnormalised (the caller divides by
