@@ -453,7 +453,8 @@ def slab_layout(shape, psf_shape, parts: int, part: int, border_quality: int = 2
 
 def release_cache(device: int = -1) -> None:
     """Free the device blocks kept for reuse by later jobs
-    (dwcu_release_cache); ``device`` < 0: every device."""
+    (``device`` < 0: every device) and the page-locked host buffers
+    (dwcu_release_cache)."""
     _check(lib().dwcu_release_cache(device))
 
 

@@ -2134,16 +2134,15 @@ int dwcu_release_cache(int32_t device)
             kv.second.clear();
         }
     }
-    if (device < 0 || !drop.empty()) {
-        copy_release();
-        std::vector<std::pair<size_t, float *>> slots;
-        {
-            std::lock_guard<std::mutex> lk(g_slot_mu);
-            slots.swap(g_slots);
-        }
-        for (auto &sl : slots) cudaFreeHost(sl.second);
-        cudaGetLastError();
+    // the host buffers serve all devices
+    copy_release();
+    std::vector<std::pair<size_t, float *>> slots;
+    {
+        std::lock_guard<std::mutex> lk(g_slot_mu);
+        slots.swap(g_slots);
     }
+    for (auto &sl : slots) cudaFreeHost(sl.second);
+    cudaGetLastError();
     int cur = 0;
     const bool had = cudaGetDevice(&cur) == cudaSuccess;
     for (auto *b : drop) {

@@ -214,9 +214,9 @@ int dwcu_job_result(dwcu_job *job, float *out, int32_t out_on_device, dwcu_opts 
  * them, at most a thirty-second of the device's memory together. */
 void dwcu_job_destroy(dwcu_job *job);
 /* Free the device blocks the library keeps for reuse on `device` (all
- * devices when negative), and with them the page-locked copy buffers and
- * error slots it keeps.  No counterpart in the reference, which allocates per
- * call. */
+ * devices when negative), and the page-locked copy buffers and error slots it
+ * keeps, which serve all devices.  No counterpart in the reference, which
+ * allocates per call. */
 int dwcu_release_cache(int32_t device);
 /* Use a caller stream (cudaStream_t) for this job's work. */
 int dwcu_job_set_stream(dwcu_job *job, void *stream);
