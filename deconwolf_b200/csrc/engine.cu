@@ -2239,12 +2239,12 @@ int dwcu_job_restore(dwcu_job *j, const float *x, const float *x_prev, const flo
     j->it.lasterror = st->lasterror;
     j->spectrum_ready = false;
     j->spec = -1;
-    if (j->flat0) {
-        // the shortcut for a constant first estimate holds for this one only
-        // if it is still that constant
-        const long long n = st->volume_elems;
-        for (long long i = 0; i < n && j->flat0; ++i) j->flat0 = x[i] == j->x0 && (!shb || x_prev[i] == j->x0);
-    }
+    j->err_due = dwcu::ErrSum{};  // of a step that failed half-way
+    // the shortcut for a constant first estimate holds for this estimate if it
+    // is that constant, whatever the job held before
+    j->flat0 = flat_first(j->g, j->s);
+    for (long long i = 0, n = st->volume_elems; i < n && j->flat0; ++i)
+        j->flat0 = x[i] == j->x0 && (!shb || x_prev[i] == j->x0);
     return DWCU_SUCCESS;
 }
 
