@@ -2158,6 +2158,10 @@ void dwcu_job_destroy(dwcu_job *j)
     if (!j) return;
     cudaSetDevice(j->s.device);
     if (j->stream) cudaStreamSynchronize(j->stream);
+    // an error's copy queued on a stream the job has left since: its slot goes
+    // to the next job
+    for (auto e : j->ev_rb)
+        if (e) cudaEventSynchronize(e);
     check_guards(j);
     if (j->graph) cudaGraphExecDestroy(j->graph);
     if (j->block) block_put(j->block);
