@@ -772,7 +772,6 @@ static int pass_x(dwcu_job *j, int op, int r2c, float2 *S, const float *src, con
     a.dst = dst;
     a.partial = j->partial;
     a.sc = j->sc;
-    a.err = &j->sc->flags;
     a.X = j->x_pitch ? j->x_pitch : g.XP;
     a.bulk = a.X % 4 == 0 && (((uintptr_t) src | (uintptr_t) srcp | (uintptr_t) j->W) & 15) == 0;
     a.GP = g.GP;

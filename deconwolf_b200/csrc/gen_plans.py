@@ -97,15 +97,6 @@ def padn(n, s):
     return n + n // s[0] + 1
 
 
-def x_fits(n):
-    """Complex half lengths the x pass takes: a CTA with one tile of rows of
-    the best split, staged with three real rows each, fits shared memory."""
-    s = best_split(n)
-    rev = (s[2], s[1], s[0]) if s[2] > 1 else (s[1], s[0], 1)
-    row = max(n + 1, padn(n, s), padn(n, rev)) | 1
-    return 64 + 8 * (row + 1) // 2 * 2 + 12 * ((2 * n + 3) // 4 * 4) + 8 * tpl_of(n, s) <= SMEM_MAX
-
-
 # Issue cost of a radix-r butterfly (about 0.65 of its real additions and
 # multiplications: pairs of them are one instruction, plus register moves)
 DFT_COST = {1: 0, 2: 4, 3: 12, 4: 12, 5: 28, 6: 32, 7: 58, 8: 38, 9: 72, 10: 66, 12: 76, 14: 128, 15: 130, 16: 112}
@@ -151,8 +142,8 @@ X_W = dict(pair=48, mid=11, op=69, sync32=9, sync=30, row=55, latency=8.8)
 
 
 def x_R(tp):
-    """Rows per tile: one CTA has at least 128 threads up to 32 threads per
-    row, two rows above (the error partials are per tile)."""
+    """Rows per tile (a CTA; the error partials are per tile): up to 32 threads
+    per row as many rows as make 128 threads, above that one."""
     return 1 if tp > 32 else 128 // tp
 
 
@@ -297,7 +288,7 @@ def main():
     args = ap.parse_args()
 
     lines_ns = supported(args.max, start=1)
-    x_ns = [n for n in supported(args.xmax) if x_fits(n)]
+    x_ns = supported(args.xmax)
     if args.only:
         keep = {int(v) for v in args.only.split(",")}
         lines_ns = [n for n in lines_ns if n in keep or n == 1]

@@ -45,7 +45,6 @@ struct XArgs {
     float *dst;            // real output (UPDATE: x_{k+1}; WEIGHTS/STORE)
     double *partial;       // per-tile error partials (ops with an error)
     const JobScalars *sc;  // bg, ...
-    int *err;              // error flags (bounded waits)
     long long X;           // real row pitch in floats (even)
     int bulk;              // real rows start at multiples of 16 bytes, X a multiple of 4
     long long GP;          // image row pitch, multiple of 4
@@ -426,7 +425,7 @@ __device__ __forceinline__ void x_row_op(const XArgs &a, int op, int t, long lon
 // A row is worked on by TP threads; in a stage of M butterflies thread t has
 // the butterflies t, t + TP, ...  TP is a power of two up to 32 -- the row
 // lies within a warp and needs no block barrier -- or a multiple of 32, where
-// the row has a barrier of its own.
+// the row has a CTA to itself.
 template <class RD, int TP>
 struct XLine {
     static constexpr int L = RD::N;
@@ -497,19 +496,18 @@ struct XCfg {
     static constexpr int MIN_BLOCKS = cmax(1, cmin(FIT_REGS, (int) (227 * 1024 / (SMEM_BYTES + 1024))));
     static_assert(THREADS % 32 == 0, "the error reduction needs full warps");
     static_assert(TP % 32 == 0 || 32 % TP == 0, "a row lies within a warp or fills whole warps");
-    static_assert(TP <= 32 || R <= 15, "one named barrier per row");
+    static_assert(TP <= 32 || R == 1, "a row of several warps has the CTA to itself");
+    static_assert(SMEM_BYTES <= 227 * 1024, "the exchange tiles fit shared memory");
 };
 
 // barrier of the threads of one row
-template <int TP, int R>
-__device__ __forceinline__ void row_sync(int row)
+template <int TP>
+__device__ __forceinline__ void row_sync()
 {
     if constexpr (TP <= 32)
         __syncwarp();
-    else if constexpr (R == 1)
-        __syncthreads();
     else
-        asm volatile("bar.sync %0, %1;" ::"r"(row + 1), "n"(TP) : "memory");
+        __syncthreads();
 }
 
 // stage twiddles applied, then the butterfly (CONJ: the conjugate twiddles)
@@ -769,12 +767,12 @@ k_xpass(XArgs a)
         if constexpr (RD::THREE) {
             float2 tm[XL::Q2][XTw<L, RB>::NB];
             x_bases<L, RA, RB, TP>(tm, t, a.twL);
-            row_sync<TP, R>(row);
+            row_sync<TP>();
             x_mid<L, RA, RB, +1, TP>(T0, T1, t, tm, XL::gap(RA, RB));
             in = T1;
         }
         x_bases<L, SL, RL, TP>(tl, t, a.twL);
-        row_sync<TP, R>(row);
+        row_sync<TP>();
 #pragma unroll
         for (int q = 0; q < QL; ++q) {
             const int j = t + q * TP;
@@ -826,7 +824,7 @@ k_xpass(XArgs a)
         float2 *F1 = F0 == T0 ? T1 : T0;
         if (a.wrapx) {
             // periodic margins of the row (see XArgs), through shared memory
-            row_sync<TP, R>(row);
+            row_sync<TP>();
             float *rowf = reinterpret_cast<float *>(T0);
 #pragma unroll
             for (int q = 0; q < QL; ++q) {
@@ -836,7 +834,7 @@ k_xpass(XArgs a)
                     for (int r = 0; r < RL; ++r) reinterpret_cast<float2 *>(rowf)[j + r * SL] = w[q][r];
                 }
             }
-            row_sync<TP, R>(row);
+            row_sync<TP>();
 #pragma unroll
             for (int q = 0; q < QL; ++q) {
                 const int j = t + q * TP;
@@ -856,7 +854,7 @@ k_xpass(XArgs a)
                     }
                 }
             }
-            row_sync<TP, R>(row);
+            row_sync<TP>();
         }
         constexpr int PK = RL % 2 == 0 ? 1 : 0;
 #pragma unroll
@@ -873,14 +871,14 @@ k_xpass(XArgs a)
         if constexpr (RD::THREE) {
             float2 tm[XL::Q2][XTw<L, RB>::NB];
             x_bases<L, RL, RB, TP>(tm, t, a.twL);
-            row_sync<TP, R>(row);
+            row_sync<TP>();
             x_mid<L, RL, RB, -1, TP>(F0, F1, t, tm, XL::gap(RL, RB));
             in = F1;
         }
         x_bases<L, M, RA, TP>(tl, t, a.twL);
 #pragma unroll
         for (int q = 0; q < XL::QP; ++q) tx[q] = __ldg(&a.tw[t + q * TP < XL::NP ? t + q * TP : 0]);
-        row_sync<TP, R>(row);
+        row_sync<TP>();
         dep_start_next();
         // last stage: both butterflies of a mirrored pair.  Butterfly M-p's
         // twiddles are W_L^{r(M-p)} = conj(w_r) e^{-2 pi i r/RA} with w_r those
