@@ -126,8 +126,10 @@ __device__ __forceinline__ float2 div_pair(float2 g, float2 d)
 // Natural logarithms of two lanes, normal and positive: q = 2^e m with m in
 // [sqrt(1/2), sqrt(2)), log q = e ln 2 + f - f^2/2 + f^3 P(f) with f = m - 1
 // and P of degree 8 fitted (weighted minimax) to that interval; ln 2 is split
-// so that e times its high part is exact.  Largest error 0.84 units in the
-// last place, mean 0.254 (0.25: correct rounding).
+// as by Cody and Waite (Software Manual for the Elementary Functions, 1980),
+// 355/512 and the rest, so that e times its high part is exact.  Over all
+// positive normal floats the largest error is 0.852 units in the last place,
+// the mean 0.25 (that of correct rounding).
 __device__ __forceinline__ float2 log_pair(float2 q)
 {
     auto both = [](float c) { return make_float2(c, c); };
@@ -485,8 +487,10 @@ struct XCfg {
     static constexpr int NKB = (L + 1 + KB - 1) / KB;
     static constexpr int THREADS = R * TP;
     static constexpr size_t ROW_BYTES = sizeof(float2) * (size_t) XL::ROW_F2;
-    // registers a thread can use without spilling (two per value held, plus
-    // twiddles, addresses and the op's operands), and the CTAs that leaves
+    // registers planned for a thread (two per value held, plus twiddles,
+    // addresses and the op's operands), and the CTAs that leaves.  Most
+    // kernels fit; a few spill 8 to 24 bytes, the ratio with a radix of 15 or
+    // 16 on the op side 200 to 430.
     static constexpr int REGS = cmin(255, cmax(48, (2 * XL::HELD + 32 + 7) / 8 * 8));
     static constexpr int FIT_REGS = cmax(1, cmin(cmin(32, 2048 / THREADS), 65536 / (REGS * THREADS)));
     // two exchange tiles per row: consecutive exchanges alternate, so each

@@ -1,5 +1,5 @@
 """The x pass on the GPU: its transforms at the edges of its thread layouts
-(4 to 192 threads per row, odd and even butterfly counts, one to three
+(4 to 256 threads per row, odd and even butterfly counts, one to three
 stages, partial row tiles) against float64, and the ratio's two routes (the
 usual range and the general one) against each other."""
 import numpy as np
