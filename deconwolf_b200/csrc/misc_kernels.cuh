@@ -194,7 +194,9 @@ k_argmax_final(const ArgmaxPartial *part, int nb, int pM, int pN, PsfPeak *out, 
         __syncthreads();
     }
     if (t == 0) {
-        const long long am = si[0], r = am / pM;
+        // (no maximum, every value NaN: any place inside the PSF will do, as
+        // the x pass reads it from there before the set-up refuses it)
+        const long long am = si[0] == LLONG_MAX ? 0 : si[0], r = am / pM;
         *out = PsfPeak{am, (int) (am % pM), (int) (r % pN), (int) (r / pN)};
         sc->psfsum = ss[0];
     }
