@@ -533,8 +533,8 @@ __device__ __forceinline__ void x_butterfly(float2 *v, const float2 (&w)[R])
 // lengths 375 / 420 / 1350: 3.9 / 4.4 / 5.5 with one value, 2.2 / 2.2 / 2.6
 // with these (largest over the 176 lengths and both directions, relative to
 // the square root of the transform's factors of two: 1.62 -> 0.86); x 2240
-// update 4.37 -> 4.45 ms, x 700 0.279 -> 0.290 (RL), whole deconvolutions
-// 0 to 1 % more.
+// update 2 to 4 % more (4.37 -> 4.45 ms, 4.20 -> 4.36 on another box), x 700
+// 4 % (RL, 0.279 -> 0.290), whole deconvolutions 0 to 1 %.
 template <int L, int RS>
 struct XTw {
     static constexpr int D = L < 128 ? (RS <= 7 ? 2 : 4) : RS <= 4 ? RS : RS <= 10 ? (RS + 1) / 2 : (RS + 2) / 3;
